@@ -100,6 +100,7 @@ struct PassArgs {
   unsigned *retry_knn;
   long long retry_cap;  // entries of retry_knn
   DeferQueue defer;
+  ClipHand hand;
   int Pb, Vb, Tb, Kb;  // caps the pass's launches hold
 };
 
@@ -300,6 +301,7 @@ __global__ void __launch_bounds__(1024) k_plan(const DiagStatic *__restrict__ ds
     a.tri_count = g.tri_count;
     a.tri_first = pa.pass == 0 ? 1 : 0;
     a.defer = pa.defer;
+    a.hand = pa.hand;
     pl.descs[d] = a;
     a.defer = DeferQueue();
     a.T_ahead = 0;
@@ -430,6 +432,7 @@ struct rpd_batch {
   int stats_variant[kKnnClasses] = {};       // first pass's neighbour variant per slot class (-1: unused)
   float stats_trial_ms[kKnnClasses][2] = {};  // the capture's trial: warp, thread (0: no trial)
   cudaEvent_t ev_probe = nullptr;  // after the probe and its compaction
+  DevBuf hand_recs, hand_ctr;  // cells handed from the octet clipping to a warp
   DevBuf retry_knn, defer_slots, defer_part, defer_fail, defer_ctr, defer_chunk_slot, work;
   DiagState *host_states = nullptr;  // pinned
   cudaGraph_t graph = nullptr;
@@ -721,6 +724,15 @@ int capture(rpd_batch *b) {
       return map_cuda(ctx, e, "alloc batch defer");
   }
   if ((e = b->work.ensure(sizeof(int))) != cudaSuccess) return map_cuda(ctx, e, "alloc batch");
+  ClipHand hand;
+  if (!any_safe) {
+    hand.capacity = clip_hand_capacity(int(cells));
+    if ((e = b->hand_recs.ensure(size_t(kClipRecordBytes) * hand.capacity)) != cudaSuccess ||
+        (e = b->hand_ctr.ensure(sizeof(int) * kClipCounters)) != cudaSuccess)
+      return map_cuda(ctx, e, "alloc batch clip records");
+    hand.recs = b->hand_recs.as<unsigned char>();
+    hand.ctr = b->hand_ctr.as<int>();
+  }
   if (!b->host_states && (e = cudaMallocHost(&b->host_states, sizeof(DiagState) * nd)) != cudaSuccess)
     return map_cuda(ctx, e, "alloc batch host");
   for (auto &x : b->ev)
@@ -855,6 +867,7 @@ int capture(rpd_batch *b) {
       if (dq.capacity < 1) dq = DeferQueue();
     }
     pa.defer = dq;
+    pa.hand = hand;
     if (j < kPassRecord && (e = mark(b->ev_pass[j])) != cudaSuccess) return fail(e, "batch event");
     if (j == 0 && nprobe) {
       // the outside probe over every seed of the probed diagrams, then the
@@ -907,6 +920,7 @@ int capture(rpd_batch *b) {
     cb.rows_plain = j == 0 ? rows_plain0 : -1;
     cb.work = b->work.as<int>();
     cb.safe = any_safe;
+    cb.hand = hand;
     if ((e = cell_batch_launch(cb, st, ctx->sm_count, &launches)) != cudaSuccess) return fail(e, "batch cells");
     // failing cells of the pass's diagrams
     k_fail_flags_batch<<<flat_blocks, 256, 0, st>>>(ds, sts, pl.rc_start, nd, b->f0.as<int>(), b->f1.as<int>());

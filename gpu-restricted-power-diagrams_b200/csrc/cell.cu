@@ -13,6 +13,7 @@ bool cell_caps_fit(int P, int V, int T, bool grid, int hc) {
 cudaError_t cell_batch_launch(const CellBatch &b, cudaStream_t st, int sm_count, int *launches) {
   if (b.ndiag <= 0) return cudaSuccess;
   if (b.safe) return cell_batch_launch_safe(b, st, sm_count, launches);
+  if (b.hand.recs) return cell_batch_launch_octet(b, st, sm_count, launches);
   if (b.P > kMaxP || b.V > kMaxV || b.T > kMaxT || b.P < 7 || b.V < 8) return cudaErrorInvalidValue;
   if (b.HC && b.defer.slots) return cudaErrorInvalidValue;  // Hessian rows are summed inline
   const Layout Lg = make_layout(b.P, b.V, b.T, true, b.HC, b.T_slot, 0, b.disjoint),
@@ -31,6 +32,7 @@ size_t defer_slot_bytes(int P, int V, int T) { return slot_bytes_for(make_layout
 
 cudaError_t cell_launch(const CellLaunch &a, cudaStream_t st, int sm_count, int *launches) {
   if (a.num <= 0) return cudaSuccess;
+  if (a.hand.recs && octet_applies(a)) return cell_launch_octet(a, st, sm_count, launches);
   if (a.precision != 0) return cell_launch_prec(a, st, sm_count, launches);
   if (a.safe_radius) return cell_launch_safe(a, st, sm_count, launches);
   if (a.P > kMaxP || a.V > kMaxV || a.T > kMaxT || a.P < 7 || a.V < 8) return cudaErrorInvalidValue;

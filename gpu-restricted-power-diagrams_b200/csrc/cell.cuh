@@ -66,6 +66,19 @@ struct DeferQueue {
   int inline_max = 16;             // cells with at most this many triangles stay inline
 };
 
+// Cells clipped with eight lanes each (clip_octet.cuh) that need a whole
+// warp from there on, as records for the launch's finish kernel.
+constexpr int kClipRecordBytes = 320;
+constexpr int kClipCounters = 3;
+struct ClipHand {
+  unsigned char *recs = nullptr;  // capacity records
+  int capacity = 0;
+  // [0] cells handed over, [1] next record to finish, [2] cells left with
+  // status kParkOverflow (no record free, or larger than the octet's caps) to
+  // be solved by the warp-per-cell kernel; zeroed before a launch
+  int *ctr = nullptr;
+};
+
 struct CellLaunch {
   const float4 *stored = nullptr;  // n seeds in stored order (reference frame)
   int n = 0;
@@ -124,6 +137,7 @@ struct CellLaunch {
   double *hess = nullptr;
   int *hessid = nullptr;
   int H = 0, HC = 1;
+  ClipHand hand;  // recs == null: clip with a warp per cell
 };
 constexpr int kParkOverflow = 101;  // internal status: the queue was full
 constexpr int kProbeMiss = 102;     // internal status: the outside probe proved nothing
@@ -145,6 +159,9 @@ size_t defer_slot_bytes(int P, int V, int T);
 cudaError_t cell_launch(const CellLaunch &a, cudaStream_t st, int sm_count = 148, int *launches = nullptr);
 // The same for a.precision > 0 (cell_prec.cu), and for FP64 clipping with
 // the weighted security-radius guard (a.safe_radius; cell_safe.cu).
+cudaError_t cell_launch_octet(const CellLaunch &a, cudaStream_t st, int sm_count, int *launches);
+// Whether a launch's cells can be clipped with eight lanes each.
+bool octet_applies(const CellLaunch &a);
 cudaError_t cell_launch_prec(const CellLaunch &a, cudaStream_t st, int sm_count, int *launches);
 cudaError_t cell_launch_safe(const CellLaunch &a, cudaStream_t st, int sm_count, int *launches);
 
@@ -204,9 +221,11 @@ struct CellBatch {
   bool safe = false;    // a diagram uses the weighted security-radius guard (its launch record decides)
   int HC = 0;           // Hessian rows' components (a diagram with rows; then no defer queue), else 0
   bool disjoint = false;  // every diagram's grid lists each triangle in one voxel (a smaller id buffer)
+  ClipHand hand;          // recs != null: clip with eight lanes per cell (the records' hand too)
 };
 cudaError_t cell_batch_launch(const CellBatch &b, cudaStream_t st, int sm_count, int *launches = nullptr);
 // The same with the guard compiled in (cell_safe.cu).
+cudaError_t cell_batch_launch_octet(const CellBatch &b, cudaStream_t st, int sm_count, int *launches);
 cudaError_t cell_batch_launch_safe(const CellBatch &b, cudaStream_t st, int sm_count, int *launches);
 
 }  // namespace rpd

@@ -259,6 +259,20 @@ __device__ __forceinline__ void trace_rec(double *tr, int cap, int lane, double 
   tr[0] = i + 1;
 }
 
+// The geometry below is written with explicit roundings (products and sums
+// fused in a fixed way), so that every kernel that computes a plane, a vertex
+// or an integral gets the same bits: cells clipped by eight lanes or by a
+// warp, alone or in a batch, in FP64 or with the float filter.
+
+// a b - c d.
+__device__ __forceinline__ double det2(double a, double b, double c, double d) {
+  return __fma_rn(a, b, -__dmul_rn(c, d));
+}
+// a x + b y + c z.
+__device__ __forceinline__ double dot3(double a, double b, double c, double x, double y, double z) {
+  return __fma_rn(a, x, __fma_rn(b, y, __dmul_rn(c, z)));
+}
+
 // Cofactor vector c of det(p1, p2, p3, e) = e . c, with the 2x2-minor
 // expansion of the reference's det4x4 (ConvexCell.cl:79-97), in double.
 __device__ __forceinline__ void cofactor(const Plane &p1, const Plane &p2, const Plane &p3, double &cx, double &cy,
@@ -266,31 +280,31 @@ __device__ __forceinline__ void cofactor(const Plane &p1, const Plane &p2, const
   const double a11 = p1.x, a21 = p1.y, a31 = p1.z, a41 = p1.w;
   const double a12 = p2.x, a22 = p2.y, a32 = p2.z, a42 = p2.w;
   const double a13 = p3.x, a23 = p3.y, a33 = p3.z, a43 = p3.w;
-  const double m12 = a21 * a12 - a11 * a22;
-  const double m13 = a31 * a12 - a11 * a32;
-  const double m14 = a41 * a12 - a11 * a42;
-  const double m23 = a31 * a22 - a21 * a32;
-  const double m24 = a41 * a22 - a21 * a42;
-  const double m34 = a41 * a32 - a31 * a42;
-  cx = m34 * a23 - m24 * a33 + m23 * a43;
-  cy = -(m34 * a13 - m14 * a33 + m13 * a43);
-  cz = m24 * a13 - m14 * a23 + m12 * a43;
-  cw = -(m23 * a13 - m13 * a23 + m12 * a33);
+  const double m12 = det2(a21, a12, a11, a22);
+  const double m13 = det2(a31, a12, a11, a32);
+  const double m14 = det2(a41, a12, a11, a42);
+  const double m23 = det2(a31, a22, a21, a32);
+  const double m24 = det2(a41, a22, a21, a42);
+  const double m34 = det2(a41, a32, a31, a42);
+  cx = dot3(m34, -m24, m23, a23, a33, a43);
+  cy = dot3(-m34, m14, -m13, a13, a33, a43);
+  cz = dot3(m24, -m14, m12, a13, a23, a43);
+  cw = dot3(-m23, m13, -m12, a13, a23, a33);
 }
 
 // Squared distance of the vertex with cofactor c from the seed (the FP64
 // clipping's cached |p|^2; the FP32 clipping reproduces it bit for bit when
 // it needs the exact value).
 __device__ __forceinline__ double vertex_d2(double cx, double cy, double cz, double cw) {
-  const double inv = 1.0 / cw;
-  const double px = cx * inv, py = cy * inv, pz = cz * inv;
-  return px * px + py * py + pz * pz;
+  const double inv = __drcp_rn(cw);
+  const double px = __dmul_rn(cx, inv), py = __dmul_rn(cy, inv), pz = __dmul_rn(cz, inv);
+  return dot3(px, py, pz, px, py, pz);
 }
 
 // e . c: the side of plane e the vertex with cofactor c lies on, scaled by
 // the cofactor (ConvexCell.cl:402-414 as e . c > 0).
 __device__ __forceinline__ double plane_side(double cx, double cy, double cz, double cw, const Plane &e) {
-  return cx * e.x + cy * e.y + cz * e.z + cw * e.w;
+  return __fma_rn(cx, e.x, __fma_rn(cy, e.y, __fma_rn(cz, e.z, __dmul_rn(cw, e.w))));
 }
 
 // Makes vertex `slot` from planes (a, b, c); false when it is degenerate.
@@ -526,29 +540,55 @@ __device__ __forceinline__ float4 plane_f(const Plane &p) {
   return make_float4(float(p.x), float(p.y), float(p.z), float(p.w));
 }
 
-// The domain box [-eps, 1000+eps]^3 as 6 planes and 8 vertices, in the
-// reference's plane order and vertex triples (ConvexCell.cl:278-308).
+// Plane i (0..5) of the domain box [-eps, 1000+eps]^3 in the reference's
+// order (ConvexCell.cl:278-298), in the frame of seed s.
+__device__ __forceinline__ Plane box_plane(float4 s, float eps, int i) {
+  const double vmin = -double(eps), vmax = 1000.0 + double(eps);
+  const double sc = i < 2 ? s.x : (i < 4 ? s.y : s.z);
+  const double sign = (i & 1) ? -1.0 : 1.0;
+  // global plane sign * x + off, off = -vmin (sign +) or vmax (sign -)
+  Plane p{0.0, 0.0, 0.0, (i & 1) ? vmax - sc : sc - vmin};
+  if (i < 2) p.x = sign;
+  else if (i < 4) p.y = sign;
+  else p.z = sign;
+  return p;
+}
+
+// Plane triple of vertex v (0..7) of the box (ConvexCell.cl:299-306).
+__device__ __forceinline__ unsigned box_vertex(int v) {
+  const unsigned cube[8] = {2u | 5u << 8 | 0u << 16, 5u | 3u << 8 | 0u << 16, 1u | 5u << 8 | 2u << 16,
+                            5u | 1u << 8 | 3u << 16, 4u | 2u << 8 | 0u << 16, 4u | 0u << 8 | 3u << 16,
+                            2u | 4u << 8 | 1u << 16, 4u | 3u << 8 | 1u << 16};
+  return cube[v];
+}
+
+// Bisector of seed s and neighbour b in the frame of s, and their squared
+// distance.  The kept side contains the seed: n = -(b - s)/|b - s|, offset of
+// the power bisector (ConvexCell.cl:321-328) or, for a wall neighbour,
+// through the neighbour itself.
+__device__ __forceinline__ Plane bisector(float4 b, float4 s, double &nd2) {
+  const double bx = double(b.x) - double(s.x), by = double(b.y) - double(s.y), bz = double(b.z) - double(s.z);
+  nd2 = dot3(bx, by, bz, bx, by, bz);
+  const double len = __dsqrt_rn(nd2), inv = __drcp_rn(len);
+  const double off = b.w <= kNoCellLimits
+                         ? len
+                         : __dmul_rn(__dadd_rn(nd2, double(b.w) - double(s.w)), __dmul_rn(0.5, inv));
+  return Plane{__dmul_rn(-bx, inv), __dmul_rn(-by, inv), __dmul_rn(-bz, inv), off};
+}
+
+// The domain box as 6 planes and 8 vertices, in the reference's plane order
+// and vertex triples (ConvexCell.cl:278-308).
 template <int PREC = 0>
 __device__ void init_box(WarpCell &w, float4 s, float eps, int lane) {
   if (lane < 6) {
-    const double vmin = -double(eps), vmax = 1000.0 + double(eps);
-    const double sc = lane < 2 ? s.x : (lane < 4 ? s.y : s.z);
-    const double sign = (lane & 1) ? -1.0 : 1.0;
-    // global plane sign * x + off, off = -vmin (sign +) or vmax (sign -)
-    const double off = (lane & 1) ? vmax - sc : sc - vmin;
-    Plane p{0.0, 0.0, 0.0, PREC == 2 ? double(float(off)) : off};
-    if (lane < 2) p.x = sign;
-    else if (lane < 4) p.y = sign;
-    else p.z = sign;
+    Plane p = box_plane(s, eps, lane);
+    if constexpr (PREC == 2) p.w = double(float(p.w));
     w.plane[lane] = p;
     if constexpr (PREC > 0) w.fpl[lane] = plane_f(p);
   }
   __syncwarp();
   if (lane < 8) {
-    const unsigned cube[8] = {2u | 5u << 8 | 0u << 16, 5u | 3u << 8 | 0u << 16, 1u | 5u << 8 | 2u << 16,
-                              5u | 1u << 8 | 3u << 16, 4u | 2u << 8 | 0u << 16, 4u | 0u << 8 | 3u << 16,
-                              2u | 4u << 8 | 1u << 16, 4u | 3u << 8 | 1u << 16};
-    const unsigned t = cube[lane];
+    const unsigned t = box_vertex(lane);
     if constexpr (PREC > 0) {
       int esc[kEscNum] = {0, 0, 0};
       make_vertex_f<PREC>(w, lane, t & 0xff, (t >> 8) & 0xff, (t >> 16) & 0xff, esc);
@@ -895,6 +935,52 @@ __device__ __noinline__ void hess_integrate(const WarpCell &w, double factor, in
   __syncwarp();
 }
 
+// The integration terms of one vertex (cofactor c, plane triple t): per
+// plane pair the two signed tets, added in a fixed order.
+__device__ __forceinline__ void integrate_vertex(const Plane *plane, unsigned t, double cx, double cy, double cz,
+                                                 double cw, double &sx, double &sy, double &sz, double &sw) {
+  const double inv = __drcp_rn(cw);
+  const double Ax = __dmul_rn(cx, inv), Ay = __dmul_rn(cy, inv), Az = __dmul_rn(cz, inv);
+  // AC = -A; projections of C on plane i: P_i = AC - (AC . n_i) n_i
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    const Plane &pi = plane[(t >> (8 * i)) & 0xff];
+    const Plane &pj = plane[(t >> (8 * ((i + 1) % 3))) & 0xff];
+    const double cxv = det2(pi.y, pj.z, pi.z, pj.y);
+    const double cyv = det2(pi.z, pj.x, pi.x, pj.z);
+    const double czv = det2(pi.x, pj.y, pi.y, pj.x);
+    const double c2 = dot3(cxv, cyv, czv, cxv, cyv, czv);
+    double Lx = 0, Ly = 0, Lz = 0;
+    if (c2 >= kVolEps2) {
+      const double k = __ddiv_rn(-dot3(Ax, Ay, Az, cxv, cyv, czv), c2);
+      Lx = __dmul_rn(k, cxv);
+      Ly = __dmul_rn(k, cyv);
+      Lz = __dmul_rn(k, czv);
+    }
+    // line i (planes i, i+1) pairs with plane i (sign -) and plane i+1
+    // (sign +): the reference's j = (i + 3 - st) % 3, w = (2 st - 1) det
+#pragma unroll
+    for (int st = 0; st < 2; ++st) {
+      const Plane &pp = st ? pj : pi;
+      const double k = dot3(Ax, Ay, Az, pp.x, pp.y, pp.z);
+      const double Px = __fma_rn(k, pp.x, -Ax), Py = __fma_rn(k, pp.y, -Ay), Pz = __fma_rn(k, pp.z, -Az);
+      const double det = dot3(Lx, -Px, -Ax, det2(Az, Py, Ay, Pz), det2(Az, Ly, Ay, Lz), det2(Py, Lz, Pz, Ly));
+      const double wt = st ? det : -det;
+      sw = __dadd_rn(sw, wt);
+      sx = __fma_rn(wt, __fma_rn(0.25, __dadd_rn(__dadd_rn(Px, Lx), -Ax), Ax), sx);
+      sy = __fma_rn(wt, __fma_rn(0.25, __dadd_rn(__dadd_rn(Py, Ly), -Ay), Ay), sy);
+      sz = __fma_rn(wt, __fma_rn(0.25, __dadd_rn(__dadd_rn(Pz, Lz), -Az), Az), sz);
+    }
+  }
+}
+
+// A cell's moments from the local frame to the global: sum w*(x_local + s) =
+// m_local + m * s.  Every kernel that writes a cell rounds alike.
+__device__ __forceinline__ double4 global_moments(const double acc[4], float4 s) {
+  const double m = acc[3];
+  return make_double4(fma(m, double(s.x), acc[0]), fma(m, double(s.y), acc[1]), fma(m, double(s.z), acc[2]), m);
+}
+
 // Signed-tet integration of the cell (ConvexCell.cl:577-619) in the local
 // frame: per vertex A and each of its planes i, the two tets (A, C, C
 // projected on plane i, C projected on the edge line of planes i, j), C the
@@ -909,40 +995,7 @@ __device__ void integrate(const WarpCell &w, double factor, double acc[4], int l
     if (s * 32 >= w.nv) break;
     const int v = s * 32 + lane;
     if (v >= w.nv) continue;
-    const double inv = 1.0 / w.cw[v];
-    const double Ax = w.cx[v] * inv, Ay = w.cy[v] * inv, Az = w.cz[v] * inv;
-    const unsigned t = w.tri[v];
-    // AC = -A; projections of C on plane i: P_i = AC - (AC . n_i) n_i
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-      const Plane &pi = w.plane[(t >> (8 * i)) & 0xff];
-      const Plane &pj = w.plane[(t >> (8 * ((i + 1) % 3))) & 0xff];
-      const double cxv = pi.y * pj.z - pi.z * pj.y;
-      const double cyv = pi.z * pj.x - pi.x * pj.z;
-      const double czv = pi.x * pj.y - pi.y * pj.x;
-      const double c2 = cxv * cxv + cyv * cyv + czv * czv;
-      double Lx = 0, Ly = 0, Lz = 0;
-      if (c2 >= kVolEps2) {
-        const double k = -(Ax * cxv + Ay * cyv + Az * czv) / c2;
-        Lx = k * cxv;
-        Ly = k * cyv;
-        Lz = k * czv;
-      }
-      // line i (planes i, i+1) pairs with plane i (sign -) and plane i+1
-      // (sign +): the reference's j = (i + 3 - st) % 3, w = (2 st - 1) det
-#pragma unroll
-      for (int st = 0; st < 2; ++st) {
-        const Plane &pp = st ? pj : pi;
-        const double k = -(Ax * pp.x + Ay * pp.y + Az * pp.z);
-        const double Px = -Ax - k * pp.x, Py = -Ay - k * pp.y, Pz = -Az - k * pp.z;
-        const double det = -Ax * (Py * Lz - Pz * Ly) - Px * (-Ay * Lz + Az * Ly) + Lx * (-Ay * Pz + Az * Py);
-        const double wt = st ? det : -det;
-        sw += wt;
-        sx += wt * (Ax + 0.25 * (Px + Lx - Ax));
-        sy += wt * (Ay + 0.25 * (Py + Ly - Ay));
-        sz += wt * (Az + 0.25 * (Pz + Lz - Az));
-      }
-    }
+    integrate_vertex(w.plane, w.tri[v], w.cx[v], w.cy[v], w.cz[v], w.cw[v], sx, sy, sz, sw);
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
@@ -953,10 +1006,10 @@ __device__ void integrate(const WarpCell &w, double factor, double acc[4], int l
   }
   const double f = factor / 6.0;
   trace_rec(tr, trcap, lane, 4, f * sx, f * sy, f * sz, f * sw, factor, w.nv, w.np);
-  acc[0] += f * sx;
-  acc[1] += f * sy;
-  acc[2] += f * sz;
-  acc[3] += f * sw;
+  acc[0] = fma(f, sx, acc[0]);
+  acc[1] = fma(f, sy, acc[1]);
+  acc[2] = fma(f, sz, acc[2]);
+  acc[3] = fma(f, sw, acc[3]);
   if constexpr (HESS) {
     if (w.harea) hess_integrate(w, factor, lane);
   }
@@ -2339,7 +2392,7 @@ __device__ __forceinline__ bool radius_reached(double d2j, double R2, double saf
 // Squared distance between two seeds, as the clipping loop computes it.
 __device__ __forceinline__ double seed_dist2(float4 b, float4 s) {
   const double bx = double(b.x) - double(s.x), by = double(b.y) - double(s.y), bz = double(b.z) - double(s.z);
-  return bx * bx + by * by + bz * bz;
+  return dot3(bx, by, bz, bx, by, bz);
 }
 
 // A cell proven outside the domain (its squared radius at most r_plain^2)
@@ -2419,11 +2472,8 @@ __device__ bool outside_certain(const WarpCell &w, const CellLaunch &a, const un
       if (c0 > i0 && i <= e) {
         // a later chunk: the lanes build its bisectors as the clipping loop does
         const float4 b = __ldg(&a.stored[__ldg(&nrow[i])]);
-        const double bx = double(b.x) - double(s.x), by = double(b.y) - double(s.y), bz = double(b.z) - double(s.z);
-        const double d2 = bx * bx + by * by + bz * bz;
-        const double len = sqrt(d2), inv = 1.0 / len;
-        const double off = b.w <= kNoCellLimits ? len : (d2 + (double(b.w) - double(s.w))) * (0.5 * inv);
-        pc = Plane{-bx * inv, -by * inv, -bz * inv, off};
+        double d2;
+        pc = bisector(b, s, d2);
       }
       bool cut = false;
       if (i > j && i <= e) {
@@ -2446,6 +2496,73 @@ __device__ bool outside_certain(const WarpCell &w, const CellLaunch &a, const un
 // cell's result does not depend on the other diagrams of its batch.
 __device__ __forceinline__ int vertex_capacity(const CellLaunch &a, const Layout &L) {
   return min(L.Vc, (a.V + 31) & ~31);
+}
+
+// A clipped cell's restriction, integration and outputs (moments, status,
+// Hessian row, used marks); outside: proven outside the domain, mass 0.
+template <int VS, bool GRID, bool INL>
+__device__ __forceinline__ void finish_cell(WarpCell &w, const CellLaunch &a, const Layout &L, float4 s, int sid,
+                                            int status, bool outside, int lane, double *tr, int trcap) {
+  const int np_cell = w.np;  // the clipped cell's planes (cone planes come after)
+  double acc[4] = {0, 0, 0, 0};
+  unsigned long long *ctr = a.counters;
+  if (outside) count(ctr, kCtrOutside, 1, lane);
+  if (status == kSuccess && !outside) {
+    if (GRID)
+      status = restrict_to_domain<VS, INL>(w, a, L, s, sid, acc, lane, ctr, tr, trcap);
+    else
+      integrate<VS, INL>(w, 1.0, acc, lane, ctr, tr, trcap);
+  }
+  if (status == kDeferred) return;  // k_cone_finish writes it
+  if (status == kParkOverflow) {
+    if (lane == 0) a.status[sid] = kParkOverflow;
+    return;
+  }
+  if (INL && a.hess && status == kSuccess) {
+    // the row (ConvexCell.cl:1133-1150): facets with a neighbour and an area
+    // above 0.2, in plane order; more than H is hessian_overflow, which
+    // keeps the moments
+    __syncwarp();
+    if (lane == 0) {
+      const int hc = a.HC, H = a.H;
+      double *hrow = a.hess + size_t(sid) * H * hc;
+      int *hids = a.hessid + size_t(sid) * H;
+      int cnt = 0;
+      for (int p = 0; p < np_cell; ++p) {
+        const double ar = w.harea[p * hc + hc - 1];
+        if (w.pnb[p] < 0 || ar <= 0.2) continue;
+        if (cnt >= H) {
+          status = kHessianOverflow;
+          break;
+        }
+        if (hc == 1) {
+          hrow[cnt] = ar;
+        } else {
+          hrow[4 * cnt + 0] = w.harea[4 * p + 0] + ar * double(s.x);
+          hrow[4 * cnt + 1] = w.harea[4 * p + 1] + ar * double(s.y);
+          hrow[4 * cnt + 2] = w.harea[4 * p + 2] + ar * double(s.z);
+          hrow[4 * cnt + 3] = ar;
+        }
+        hids[cnt] = w.pnb[p];
+        ++cnt;
+      }
+      if (status == kSuccess && cnt < H) hids[cnt] = -1;
+    }
+    status = __shfl_sync(kFull, status, 0);
+  }
+  if (lane == 0) {
+    a.status[sid] = status;
+    if (status == kSuccess || status == kHessianOverflow)
+      a.out[sid] = global_moments(acc, s);
+    else
+      a.out[sid] = make_double4(0.0, 0.0, 0.0, 0.0);
+  }
+  if (GRID && a.used && status == kSuccess && acc[3] >= a.keep_volume) {
+    // a used cell (ConvexCell.cl:1118-1126)
+    if (lane == 0) *(volatile unsigned char *)&a.used[sid] = 1;
+    __syncwarp();
+    if (a.mark_dist >= 1) mark_neighbours(a.used, w.tri, w.nv, w.pnb, 1, lane, 32);
+  }
 }
 
 // One row of a cell launch (one warp): clip, restrict, integrate, write.
@@ -2485,7 +2602,6 @@ __device__ __forceinline__ void cell_row(const CellLaunch &a, const Layout &L, u
   const int trcap = a.trace_cap;
   trace_rec(tr, trcap, lane, 0, s.x, s.y, s.z, s.w, sid);
   int status = kSuccess;
-  double acc[4] = {0, 0, 0, 0};
   if (s.w <= kNoCellLimits) {
     if (lane == 0) {
       a.status[sid] = kSuccess;
@@ -2540,15 +2656,7 @@ __device__ __forceinline__ void cell_row(const CellLaunch &a, const Layout &L, u
       const unsigned z = __ldg(&nrow[i]);
       zl = z;
       if (z != kNone) {
-        const float4 b = __ldg(&a.stored[z]);
-        const double bx = double(b.x) - double(s.x), by = double(b.y) - double(s.y), bz = double(b.z) - double(s.z);
-        nd2 = bx * bx + by * by + bz * bz;
-        const double len = sqrt(nd2), inv = 1.0 / len;
-        // kept side contains the seed: n = -(b - s)/|b - s|, offset of the
-        // power bisector (ConvexCell.cl:321-328) or, for a wall neighbour,
-        // through the neighbour itself
-        const double off = b.w <= kNoCellLimits ? len : (nd2 + (double(b.w) - double(s.w))) * (0.5 * inv);
-        pl = Plane{-bx * inv, -by * inv, -bz * inv, off};
+        pl = bisector(__ldg(&a.stored[z]), s, nd2);
         if constexpr (PREC == 2) pl = Plane{double(float(pl.x)), double(float(pl.y)), double(float(pl.z)), double(float(pl.w))};
         valid = true;
       }
@@ -2660,7 +2768,6 @@ __device__ __forceinline__ void cell_row(const CellLaunch &a, const Layout &L, u
   }
   if (status == kSuccess && !reached && !exhausted && !outside) status = kSecurityRadiusNotReached;
   if (status == kSuccess && out_known) outside = true;
-  const int np_cell = w.np;  // the clipped cell's planes (cone planes come after)
   if (a.border_d > 0) {
     // bordering pass (ConvexCell.cl:756-809): the clipped cell marks its
     // neighbours; statuses and moments stay those of the main passes
@@ -2668,65 +2775,7 @@ __device__ __forceinline__ void cell_row(const CellLaunch &a, const Layout &L, u
     if (status == kSuccess) mark_neighbours(a.used, w.tri, w.nv, w.pnb, a.border_d, lane, 32);
     return;
   }
-  if (outside) count(ctr, kCtrOutside, 1, lane);
-  if (status == kSuccess && !outside) {
-    if (GRID)
-      status = restrict_to_domain<VS, INL>(w, a, L, s, sid, acc, lane, ctr, tr, trcap);
-    else
-      integrate<VS, INL>(w, 1.0, acc, lane, ctr, tr, trcap);
-  }
-  if (status == kDeferred) return;  // k_cone_finish writes it
-  if (status == kParkOverflow) {
-    if (lane == 0) a.status[sid] = kParkOverflow;
-    return;
-  }
-  if (INL && a.hess && status == kSuccess) {
-    // the row (ConvexCell.cl:1133-1150): facets with a neighbour and an area
-    // above 0.2, in plane order; more than H is hessian_overflow, which
-    // keeps the moments
-    __syncwarp();
-    if (lane == 0) {
-      const int hc = a.HC, H = a.H;
-      double *hrow = a.hess + size_t(sid) * H * hc;
-      int *hids = a.hessid + size_t(sid) * H;
-      int cnt = 0;
-      for (int p = 0; p < np_cell; ++p) {
-        const double ar = w.harea[p * hc + hc - 1];
-        if (w.pnb[p] < 0 || ar <= 0.2) continue;
-        if (cnt >= H) {
-          status = kHessianOverflow;
-          break;
-        }
-        if (hc == 1) {
-          hrow[cnt] = ar;
-        } else {
-          hrow[4 * cnt + 0] = w.harea[4 * p + 0] + ar * double(s.x);
-          hrow[4 * cnt + 1] = w.harea[4 * p + 1] + ar * double(s.y);
-          hrow[4 * cnt + 2] = w.harea[4 * p + 2] + ar * double(s.z);
-          hrow[4 * cnt + 3] = ar;
-        }
-        hids[cnt] = w.pnb[p];
-        ++cnt;
-      }
-      if (status == kSuccess && cnt < H) hids[cnt] = -1;
-    }
-    status = __shfl_sync(kFull, status, 0);
-  }
-  if (lane == 0) {
-    a.status[sid] = status;
-    // local moments -> global: sum w*(x_local + s) = m_local + m * s
-    const double m = acc[3];
-    if (status == kSuccess || status == kHessianOverflow)
-      a.out[sid] = make_double4(acc[0] + m * double(s.x), acc[1] + m * double(s.y), acc[2] + m * double(s.z), m);
-    else
-      a.out[sid] = make_double4(0.0, 0.0, 0.0, 0.0);
-  }
-  if (used_on && status == kSuccess && acc[3] >= a.keep_volume) {
-    // a used cell (ConvexCell.cl:1118-1126)
-    if (lane == 0) *(volatile unsigned char *)&a.used[sid] = 1;
-    __syncwarp();
-    if (a.mark_dist >= 1) mark_neighbours(a.used, w.tri, w.nv, w.pnb, 1, lane, 32);
-  }
+  finish_cell<VS, GRID, INL>(w, a, L, s, sid, status, outside, lane, tr, trcap);
 }
 
 template <int VS, bool GRID, bool INL, int PREC = 0, int SAFE = 0>
@@ -2878,11 +2927,8 @@ __device__ __forceinline__ void probe_row(const ProbeLaunch &p, const Layout &L,
       const bool valid = best != kEmptyKey && __uint_as_float(unsigned(best >> 32)) <= max_d2;
       if (valid) {
         const float4 b = __ldg(&p.stored[unsigned(best & 0xffffffffull)]);
-        const double bx = double(b.x) - double(s.x), by = double(b.y) - double(s.y), bz = double(b.z) - double(s.z);
-        const double nd2 = bx * bx + by * by + bz * bz;
-        const double len = sqrt(nd2), inv = 1.0 / len;
-        const double off = b.w <= kNoCellLimits ? len : (nd2 + (double(b.w) - double(s.w))) * (0.5 * inv);
-        pl = Plane{-bx * inv, -by * inv, -bz * inv, off};
+        double nd2;
+        pl = bisector(b, s, nd2);
       }
       const int nb = __popc(__ballot_sync(kFull, valid));
       init_box(w, s, p.cube_eps, lane);
@@ -2932,9 +2978,9 @@ __global__ void __launch_bounds__(128, 6) k_probe_batch(const ProbeLaunch *__res
 
 // Rows of many diagrams in one persistent launch (batched solves): diagram
 // d owns rows start[d] .. start[d+1] and its own launch record descs[d];
-// warps stride over the rows.  park_counter (optional): the re-run of the
-// cells that found the defer queue full, which exits unless the queue
-// overflowed.
+// warps stride over the rows.  park_counter, left (optional): the re-run of
+// the cells that found the defer queue full or that the octet clipping left
+// (ClipHand::ctr[2]), which exits when there are none.
 // work (optional, zeroed before the launch): warps take their rows one at a
 // time from this counter (persistent launches of unknown row counts, so a
 // warp that drew heavy rows does not hold the launch back); null: warp w
@@ -2943,9 +2989,9 @@ template <int VS, bool GRID, bool INL, int SAFE = 0>
 __global__ void __launch_bounds__(128, 5)
     k_cell_batch(const CellLaunch *__restrict__ descs, const int *__restrict__ start, int ndiag,
                  const __grid_constant__ Layout L, int only_status, const int *__restrict__ park_counter,
-                 int park_capacity, int *__restrict__ work) {
+                 int park_capacity, const int *__restrict__ left, int *__restrict__ work) {
   extern __shared__ __align__(16) unsigned char smem[];
-  if (park_counter && *park_counter <= park_capacity) return;
+  if ((park_counter || left) && !(park_counter && *park_counter > park_capacity) && !(left && *left > 0)) return;
   const int lane = threadIdx.x & 31;
   unsigned char *wsmem = smem + size_t(threadIdx.x >> 5) * L.total;
   const int total = start[ndiag];
@@ -3102,11 +3148,8 @@ __device__ __forceinline__ void finish_slot(const DeferQueue &dq, const Layout &
   }
   const float4 s = a.stored[sid];
   a.status[sid] = status;
-  const double m = acc[3];
-  a.out[sid] = status == kSuccess
-                   ? make_double4(acc[0] + m * double(s.x), acc[1] + m * double(s.y), acc[2] + m * double(s.z), m)
-                   : make_double4(0.0, 0.0, 0.0, 0.0);
-  if (a.used && status == kSuccess && m >= a.keep_volume) {
+  a.out[sid] = status == kSuccess ? global_moments(acc, s) : make_double4(0.0, 0.0, 0.0, 0.0);
+  if (a.used && status == kSuccess && acc[3] >= a.keep_volume) {
     // a used cell (ConvexCell.cl:1118-1126), marked from the parked copy
     *(volatile unsigned char *)&a.used[sid] = 1;
     if (a.mark_dist >= 1) {
@@ -3171,6 +3214,23 @@ int warps_per_block_for(const Layout &L) {
   return w;
 }
 
+// The cone kernels over the cells a launch parked, and their reduction.
+template <int VS>
+cudaError_t launch_cones(const CellLaunch &a, const Layout &L, cudaStream_t st, int sm_count, int *launches) {
+  const int warps_per_block = warps_per_block_for(L);
+  if (warps_per_block == 0) return cudaErrorInvalidValue;
+  const size_t smem = size_t(L.total) * warps_per_block;
+  cudaError_t e;
+  if ((e = allow_smem(reinterpret_cast<const void *>(k_cone<VS, kConeInner>), smem)) != cudaSuccess ||
+      (e = allow_smem(reinterpret_cast<const void *>(k_cone<VS, kConeCorner>), smem)) != cudaSuccess)
+    return e;
+  k_cone<VS, kConeInner><<<sm_count * 4, warps_per_block * 32, smem, st>>>(a, L);
+  k_cone<VS, kConeCorner><<<sm_count * 4, warps_per_block * 32, smem, st>>>(a, L);
+  k_cone_finish<<<(a.defer.capacity + 127) / 128, 128, 0, st>>>(a, L);
+  if (launches) *launches += 3;
+  return cudaGetLastError();
+}
+
 template <int VS, int PREC = 0, int SAFE = 0>
 cudaError_t launch_vs(const CellLaunch &a, const Layout &L, cudaStream_t st, int sm_count, int *launches) {
   const int warps_per_block = warps_per_block_for(L);
@@ -3184,13 +3244,8 @@ cudaError_t launch_vs(const CellLaunch &a, const Layout &L, cudaStream_t st, int
     if (e != cudaSuccess) return e;
     k_cell<VS, true, false, PREC, SAFE><<<blocks, warps_per_block * 32, smem, st>>>(a, L);
     if (a.after_cell) cudaEventRecord(a.after_cell, st);
-    if ((e = allow_smem(reinterpret_cast<const void *>(k_cone<VS, kConeInner>), smem)) != cudaSuccess ||
-        (e = allow_smem(reinterpret_cast<const void *>(k_cone<VS, kConeCorner>), smem)) != cudaSuccess)
-      return e;
-    k_cone<VS, kConeInner><<<sm_count * 4, warps_per_block * 32, smem, st>>>(a, L);
-    k_cone<VS, kConeCorner><<<sm_count * 4, warps_per_block * 32, smem, st>>>(a, L);
-    k_cone_finish<<<(a.defer.capacity + 127) / 128, 128, 0, st>>>(a, L);
-    if (launches) *launches += 4;
+    if (launches) ++*launches;
+    return launch_cones<VS>(a, L, st, sm_count, launches);
   } else if (a.grid.size > 0) {
     e = allow_smem(reinterpret_cast<const void *>(k_cell<VS, true, true, PREC, SAFE>), smem);
     if (e != cudaSuccess) return e;
@@ -3222,7 +3277,7 @@ int resident_blocks(Kernel k, int threads, size_t smem, int sm_count) {
 template <int VS, bool GRID, bool INL, int SAFE = 0>
 cudaError_t batch_cells(const CellLaunch *descs, const int *start, int ndiag, const Layout &L, int only_status,
                         const int *park_counter, int park_capacity, long rows, int *work, cudaStream_t st,
-                        int sm_count) {
+                        int sm_count, const int *left = nullptr) {
   const int wpb = warps_per_block_for(L);
   if (wpb == 0) return cudaErrorInvalidValue;
   const size_t smem = size_t(L.total) * wpb;
@@ -3237,13 +3292,31 @@ cudaError_t batch_cells(const CellLaunch *descs, const int *start, int ndiag, co
     blocks = resident_blocks(k, wpb * 32, smem, sm_count);
     if (work && (e = cudaMemsetAsync(work, 0, sizeof(int), st)) != cudaSuccess) return e;
   }
-  k<<<blocks, wpb * 32, smem, st>>>(descs, start, ndiag, L, only_status, park_counter, park_capacity, work);
+  k<<<blocks, wpb * 32, smem, st>>>(descs, start, ndiag, L, only_status, park_counter, park_capacity, left, work);
   return cudaGetLastError();
 }
 
 cudaError_t record_after_cell(const CellBatch &b, cudaStream_t st) {
   // an event node when the stream is being captured
   return b.after_cell ? cudaEventRecordWithFlags(b.after_cell, st, cudaEventRecordExternal) : cudaSuccess;
+}
+
+// The cone kernels over the cells a batched launch parked.
+template <int VS>
+cudaError_t launch_cones_batch(const CellBatch &b, const Layout &Lg, cudaStream_t st, int sm_count) {
+  const int wpb = warps_per_block_for(Lg);
+  if (wpb == 0) return cudaErrorInvalidValue;
+  const size_t smem = size_t(Lg.total) * wpb;
+  auto ki = k_cone_batch<VS, kConeInner>;
+  auto kr = k_cone_batch<VS, kConeCorner>;
+  cudaError_t e;
+  if ((e = allow_smem(reinterpret_cast<const void *>(ki), smem)) != cudaSuccess ||
+      (e = allow_smem(reinterpret_cast<const void *>(kr), smem)) != cudaSuccess)
+    return e;
+  ki<<<resident_blocks(ki, wpb * 32, smem, sm_count), wpb * 32, smem, st>>>(b.descs, b.defer, Lg);
+  kr<<<resident_blocks(kr, wpb * 32, smem, sm_count), wpb * 32, smem, st>>>(b.descs, b.defer, Lg);
+  k_cone_finish_batch<<<sm_count * 4, 128, 0, st>>>(b.descs, b.defer, Lg);
+  return cudaGetLastError();
 }
 
 template <int VS, int SAFE = 0>
@@ -3270,16 +3343,7 @@ cudaError_t launch_batch_vs(const CellBatch &b, const Layout &Lg, const Layout &
                                         sm_count)) != cudaSuccess)
     return e;
   if ((e = record_after_cell(b, st)) != cudaSuccess) return e;
-  const int wpb = warps_per_block_for(Lg);
-  const size_t smem = size_t(Lg.total) * wpb;
-  auto ki = k_cone_batch<VS, kConeInner>;
-  auto kr = k_cone_batch<VS, kConeCorner>;
-  if ((e = allow_smem(reinterpret_cast<const void *>(ki), smem)) != cudaSuccess ||
-      (e = allow_smem(reinterpret_cast<const void *>(kr), smem)) != cudaSuccess)
-    return e;
-  ki<<<resident_blocks(ki, wpb * 32, smem, sm_count), wpb * 32, smem, st>>>(b.descs, b.defer, Lg);
-  kr<<<resident_blocks(kr, wpb * 32, smem, sm_count), wpb * 32, smem, st>>>(b.descs, b.defer, Lg);
-  k_cone_finish_batch<<<sm_count * 4, 128, 0, st>>>(b.descs, b.defer, Lg);
+  if ((e = launch_cones_batch<VS>(b, Lg, st, sm_count)) != cudaSuccess) return e;
   if ((e = batch_cells<VS, true, true, SAFE>(b.descs_inline, b.start_grid, b.ndiag, Lg, kParkOverflow, b.defer.counters,
                                        b.defer.capacity, -1, b.work, st, sm_count)) != cudaSuccess)
     return e;

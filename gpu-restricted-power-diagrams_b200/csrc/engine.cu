@@ -420,6 +420,13 @@ int knn_variant_for(rpd_solver *s, const int *ids, int num, int K, unsigned *out
   return ctx->knn_variant[K];
 }
 
+// Launches of fewer rows clip with a warp per cell: an octet's cell takes
+// longer than a warp's, which only more cells at a time repay (uniform seeds,
+// K 50, octet / warp: 2,000 rows 0.102 / 0.076 ms in the box and 0.145 /
+// 0.122 in a cube domain, 4,000 rows 0.109 / 0.127 and 0.156 / 0.189, 16,000
+// rows 0.205 / 0.377 and 0.295 / 0.547).
+constexpr int kOctetMinRows = 4096;
+
 // One pass (VoroAlgoComputeData::launch, voronoi.cpp:861-1036): the K
 // nearest of the listed seeds, then their cells with this pass's caps.
 static_assert(int(RPD_CTR_NUM) == int(kCtrNum), "counter enums out of sync");
@@ -518,17 +525,30 @@ int run_pass(rpd_solver *s, const int *ids, int num, int K, int P, int V, int T,
     dq.fail = s->defer_fail.as<int>();
     dq.counters = s->defer_ctr.as<int>();
   }
+  if (num >= kOctetMinRows && octet_applies(a)) {
+    ClipHand &hd = a.hand;
+    hd.capacity = clip_hand_capacity(num);
+    if ((e = s->hand_recs.ensure(size_t(kClipRecordBytes) * hd.capacity)) != cudaSuccess ||
+        (e = s->hand_ctr.ensure(sizeof(int) * kClipCounters)) != cudaSuccess)
+      return map_cuda(ctx, e, "alloc clip records");
+    cudaMemsetAsync(s->hand_ctr.ptr, 0, sizeof(int) * kClipCounters, st);
+    hd.recs = s->hand_recs.as<unsigned char>();
+    hd.ctr = s->hand_ctr.as<int>();
+  }
   int launches = 0;
   if ((e = cell_launch(a, st, ctx->sm_count, &launches)) != cudaSuccess) return map_cuda(ctx, e, "cell kernel");
-  if (a.defer.slots) {
-    // cells that found the queue full run again with their cones inline
-    int ctrs[kDeferCounters] = {};
-    cudaMemcpyAsync(ctrs, a.defer.counters, sizeof(ctrs), cudaMemcpyDeviceToHost, st);
+  if (a.defer.slots || a.hand.recs) {
+    // cells that found a queue full, or larger than the octet clipping
+    // holds, run again with a warp each and their cones inline
+    int ctrs[kDeferCounters] = {}, hctr[kClipCounters] = {};
+    if (a.defer.slots) cudaMemcpyAsync(ctrs, a.defer.counters, sizeof(ctrs), cudaMemcpyDeviceToHost, st);
+    if (a.hand.recs) cudaMemcpyAsync(hctr, a.hand.ctr, sizeof(hctr), cudaMemcpyDeviceToHost, st);
     if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return map_cuda(ctx, e, "cell kernel");
     const int parked = ctrs[0];
     if (a.T_ahead > 0) s->ahead_max = ctrs[3];
-    if (parked > a.defer.capacity) {
+    if (parked > a.defer.capacity || hctr[2] > 0) {
       CellLaunch b = a;
+      b.hand = ClipHand();
       b.defer = DeferQueue();
       b.T_ahead = 0;
       b.only_status = kParkOverflow;
@@ -1410,6 +1430,8 @@ void solver_trim(rpd_solver *s) {
   s->defer_fail.release();
   s->defer_ctr.release();
   s->defer_chunk_slot.release();
+  s->hand_recs.release();
+  s->hand_ctr.release();
   s->hess.release();  // --hessian rows are read out before a trim
   s->hessid.release();
   s->hess_h = 0;
@@ -1420,11 +1442,13 @@ size_t solver_device_bytes(const rpd_solver *s) {
                        &s->ring_bound, &s->knn, &s->knn_part, &s->tri_count, &s->knn_user, &s->counter64, &s->g_flags, &s->g_points,
                        &s->g_tris, &s->g_list, &s->g_offsets, &s->g_sat, &s->g_tsat, &s->out, &s->status, &s->ids_a, &s->ids_b,
                        &s->ids_c, &s->fail_ws, &s->hist, &s->gather, &s->defer_slots, &s->defer_part, &s->defer_fail,
-                       &s->defer_ctr, &s->defer_chunk_slot, &s->wmin, &s->used, &s->hess, &s->hessid};
+                       &s->defer_ctr, &s->defer_chunk_slot, &s->hand_recs, &s->hand_ctr, &s->wmin, &s->used, &s->hess, &s->hessid};
   size_t t = 0;
   for (const DevBuf *x : b) t += x->bytes;
   return t;
 }
+
+int clip_hand_capacity(int num) { return std::min(num, 65536 + num / 8); }
 
 int t_ahead_cap(int P, int K, int T, int max_extra) {
   int T_ahead = 0;

@@ -101,6 +101,7 @@ struct rpd_solver {
   rpd::DevBuf hist;            // int[16]: status histogram + counts
   rpd::DevBuf gather;          // user-order staging for outputs
   rpd::DevBuf defer_slots, defer_part, defer_fail, defer_ctr, defer_chunk_slot;  // parked boundary cells
+  rpd::DevBuf hand_recs, hand_ctr;  // cells handed from the octet clipping to a warp
   int ahead_max = 0;           // the largest triangle count the first pass parked ahead
   bool have_results = false;
   bool use_defer = true;       // park heavy boundary cells for the chunked kernel
@@ -132,5 +133,8 @@ void solver_trim(rpd_solver *s);
 // stop once P or K (assumed to grow in every pass) outgrow their limits
 // (voronoi.cpp:867); 0 when no retry surely runs.
 int t_ahead_cap(int P, int K, int T, int max_extra);
+// Records for the clipped cells of a launch that need a warp: its boundary
+// cells, whose share falls as the cell count grows.
+int clip_hand_capacity(int num);
 
 }  // namespace rpd
