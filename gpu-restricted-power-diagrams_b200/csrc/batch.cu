@@ -708,7 +708,7 @@ int capture(rpd_batch *b) {
     return map_cuda(ctx, e, "alloc batch knn");
   // parked boundary cells: one queue for the batch, its bytes fixed by the
   // first pass; later passes (larger slots) hold fewer cells
-  const int chunk = 32;  // the cone kernels' chunk (a warp's lanes take one triangle each)
+  const int chunk = kConeChunk;
   const int cap0 = int(std::min<long long>(cells, std::max<long long>(32768, cells / 8)));
   // the first pass's slots hold the triangle overflows parked ahead
   int Tslot0 = Tb[0];

@@ -45,6 +45,10 @@ enum CellCounter {
   kCtrNum
 };
 
+// Triangles of one work item of the cone kernels; a cell's sum adds its
+// chunks' sums in order, also where a cell's own warp takes them all.
+constexpr int kConeChunk = 16;
+
 // Boundary cells with many triangles park their clipped cell here; a second
 // kernel spreads their triangles over all warps in chunks.
 struct DeferQueue {
@@ -62,7 +66,7 @@ struct DeferQueue {
   double *part = nullptr;          // capacity * max_chunks * 4 partial moments, by work item
   int *fail = nullptr;             // capacity * max_chunks: (triangle << 4) | status, or INT_MAX
   int max_chunks = 0;              // ceil(T / chunk)
-  int chunk = 32;                  // triangles per work item
+  int chunk = kConeChunk;          // triangles per work item
   int inline_max = 16;             // cells with at most this many triangles stay inline
 };
 

@@ -91,6 +91,9 @@ __host__ __device__ inline Layout make_layout(int P, int V, int T, bool grid, in
   L.prec = prec;
   L.Pc = (P + 3) & ~3;
   L.Vc = (V + 31) & ~31;
+  // the cone kernels keep their lists in the vertex arrays (ConeOct,
+  // ConeLists) and parked cells their faces in two of them
+  while (grid && ((L.Vc < 64 && L.Pc > 76) || 2 * (L.Pc + 1) > 5 * L.Vc)) L.Vc += 32;
   L.G = grid ? (disjoint ? (T + 31) & ~31 : pow2_at_least(2 * T)) : 0;
   L.Mw = (L.Pc + 31) / 32;
   L.T = T > t_slot ? T : t_slot;
@@ -1507,21 +1510,30 @@ __device__ int drop_separated(const WarpCell &w, const DevGrid &g, float4 s, int
 // outward normal, of the signed tetrahedra (a, c, u, v), c any point of G's
 // plane.  The sides pass through a and give nothing.  Every edge is a
 // segment clipped by a few planes, so a piece needs neither 3D clipping nor
-// polygon buffers: one triangle per lane, registers only.  Equal to the
-// reference's clipped-cone integral (ConvexCell.cl:1082-1115) in exact
-// arithmetic.
-constexpr int kFaceCap = 64;  // faces of one cell culled per batch of a 64-bit mask
+// polygon buffers.  Equal to the reference's clipped-cone integral
+// (ConvexCell.cl:1082-1115) in exact arithmetic.
+//
+// Eight lanes per triangle, four triangles at a time: the lanes classify the
+// cell's vertices against the cone's four planes and list the edges to clip
+// -- the faces' edges that may meet the cone, the cone planes' lines in the
+// faces that they cut -- in one list of the warp, whose entries the 32 lanes
+// then take.  One lane per triangle, the form before, kept 10 of 32 lanes
+// busy (the triangles' faces and cuts differ) and took 200 us for one work
+// item, the whole launch of a small diagram; now 18 of 32 and 100 us.  Clip
+// bounds are compared as fractions, so that a segment costs two divisions
+// and not one per plane.  Measured, cone kernels of the first pass: 250K
+// uniform seeds in a cube 2.5 -> 1.5 ms, 2M blue noise (second pass) 5.6 ->
+// 2.2 ms, 1M lattice seeds in a blob 2.8 -> 2.3 ms; 59K cells with Hessian
+// rows, cones in the cell's own warp, 5.8 -> 3.1 ms.  What bounds it: the
+// latency of FP64 chains (IPC 1.8 of 4; five and six blocks per SM instead of
+// four change nothing).
+
+// The plane across edge i of face f (i counted as in the face's vertex list).
+__device__ __forceinline__ unsigned char *face_nb(const WarpCell &w) { return reinterpret_cast<unsigned char *>(w.edge); }
 
 // Face lists of the cell, each counter-clockwise around the face's outward
 // normal (-n of its plane), and vertex positions (local frame) in px/py/pz.
-// Angular bounds of the faces seen from the apex: per face, the unit axis
-// and the half-angle (with cos, sin) of a cone from a that holds the face,
-// as floats in the backup arrays (unused on this path); kAngFaces faces fit.
-__device__ __forceinline__ float *face_angles(const WarpCell &w) { return reinterpret_cast<float *>(w.bcw); }
-__device__ __forceinline__ int face_angle_cap(const WarpCell &w) { return (20 * w.vc) / 24; }
-__device__ __forceinline__ unsigned char *face_nb(const WarpCell &w) { return reinterpret_cast<unsigned char *>(w.edge); }
-
-__device__ void build_faces(const WarpCell &w, double *px, double *py, double *pz, const double a[3], int lane) {
+__device__ void build_faces(const WarpCell &w, double *px, double *py, double *pz, int lane) {
   const int np = w.np, nv = w.nv;
   int *fstart = w.fstart;
   unsigned char *fv = w.fv;
@@ -1604,193 +1616,111 @@ __device__ void build_faces(const WarpCell &w, double *px, double *py, double *p
       }
       nb[f0 + i] = (unsigned char)e;
     }
-    if (p < face_angle_cap(w)) {
-      float *ang = face_angles(w) + 6 * p;
-      float ux = 0.f, uy = 0.f, uz = 0.f;
-      for (int i = 0; i < k; ++i) {
-        const int v = fv[f0 + i];
-        const float dx = float(px[v] - a[0]), dy = float(py[v] - a[1]), dz = float(pz[v] - a[2]);
-        const float il = rsqrtf(fmaxf(dx * dx + dy * dy + dz * dz, 1e-30f));
-        ux += dx * il;
-        uy += dy * il;
-        uz += dz * il;
-      }
-      const float ul = rsqrtf(fmaxf(ux * ux + uy * uy + uz * uz, 1e-30f));
-      ux *= ul;
-      uy *= ul;
-      uz *= ul;
-      float cmin = 1.f;
-      for (int i = 0; i < k; ++i) {
-        const int v = fv[f0 + i];
-        const float dx = float(px[v] - a[0]), dy = float(py[v] - a[1]), dz = float(pz[v] - a[2]);
-        const float il = rsqrtf(fmaxf(dx * dx + dy * dy + dz * dz, 1e-30f));
-        cmin = fminf(cmin, (dx * ux + dy * uy + dz * uz) * il);
-      }
-      const float th = acosf(fmaxf(-1.f, fminf(1.f, cmin)));
-      ang[0] = ux;
-      ang[1] = uy;
-      ang[2] = uz;
-      ang[3] = th;
-      ang[4] = cosf(th);
-      ang[5] = sinf(th);
-    }
   }
   __syncwarp();
 }
 
-struct ConePiece {
-  double a[3];      // apex
-  double c[4][4];   // side planes (through a) and the triangle's plane, inside >= 0
-  double t[3][3];   // triangle corners, counter-clockwise around c[3]
-  double acc[4];    // sum of w*x, w*y, w*z, w (unscaled: 6x the volume)
+// Work space of one octet: the cone of its triangle.  It lies, with the
+// octet's marks, in the vertex arrays (not used with an inner apex), the
+// warp's list of tasks in the backup's.
+struct ConeOct {
+  double c[4][4];  // side planes (through a) and the triangle's plane, inside >= 0
+  double t[3][3];  // triangle corners, counter-clockwise around c[3]
 };
+constexpr int kConeTasks = 128;  // octet << 24 | face << 16 | edge, or ... | 0x8000 | cone plane
 
 __device__ __forceinline__ double pval(const double *n, double x, double y, double z) {
-  return fma(n[0], x, fma(n[1], y, fma(n[2], z, n[3])));
+  return __fma_rn(n[0], x, __fma_rn(n[1], y, __fma_rn(n[2], z, n[3])));
 }
 
-// Signed tetrahedron (a, c, u, v) into acc: 6 * volume and 6 * volume * 4 * centroid.
-__device__ __forceinline__ void edge_tet(ConePiece &q, const double c[3], const double u[3], const double v[3]) {
-  const double cx = c[0] - q.a[0], cy = c[1] - q.a[1], cz = c[2] - q.a[2];
-  const double ux = u[0] - q.a[0], uy = u[1] - q.a[1], uz = u[2] - q.a[2];
-  const double vx = v[0] - q.a[0], vy = v[1] - q.a[1], vz = v[2] - q.a[2];
-  const double det = cx * (uy * vz - uz * vy) - cy * (ux * vz - uz * vx) + cz * (ux * vy - uy * vx);
-  q.acc[0] += det * (q.a[0] + c[0] + u[0] + v[0]);
-  q.acc[1] += det * (q.a[1] + c[1] + u[1] + v[1]);
-  q.acc[2] += det * (q.a[2] + c[2] + u[2] + v[2]);
-  q.acc[3] += det * 4.0;
-}
-
-// Clips segment u + s (v - u), s in [lo, hi], by plane n (inside >= 0).
-__device__ __forceinline__ void clip_seg(double eu, double ev, double &lo, double &hi) {
-  if (eu >= 0.0 && ev >= 0.0) return;
-  if (eu < 0.0 && ev < 0.0) {
-    hi = -1.0;
-    return;
+// A segment's parameter range [ln/ld, hn/hd], denominators positive.
+struct Span {
+  double ln, ld, hn, hd;
+  __device__ __forceinline__ void lower(double n, double d) {
+    if (n * ld > ln * d) {
+      ln = n;
+      ld = d;
+    }
   }
-  const double s = eu / (eu - ev);
-  if (eu < 0.0) lo = fmax(lo, s);
-  else hi = fmin(hi, s);
-}
+  __device__ __forceinline__ void upper(double n, double d) {
+    if (n * hd < hn * d) {
+      hn = n;
+      hd = d;
+    }
+  }
+  // clips the line x0 + s d by plane n
+  __device__ __forceinline__ void clip_line(const double *n, const double x0[3], const double d[3]) {
+    const double v0 = pval(n, x0[0], x0[1], x0[2]);
+    const double sl = dot3(n[0], n[1], n[2], d[0], d[1], d[2]);
+    if (sl > 0.0) lower(-v0, sl);
+    else if (sl < 0.0) upper(v0, -sl);
+    else if (v0 < 0.0) upper(-1e200, 1.0);
+  }
+  __device__ __forceinline__ bool open() const { return ln * hd < hn * ld; }
+};
 
 // Line of planes n1 and n2 (inside >= 0 each) as x0 + s d with d = n1 x n2;
 // false when they are parallel.
 __device__ __forceinline__ bool plane_line(const double *n1, const double *n2, double x0[3], double d[3]) {
-  d[0] = n1[1] * n2[2] - n1[2] * n2[1];
-  d[1] = n1[2] * n2[0] - n1[0] * n2[2];
-  d[2] = n1[0] * n2[1] - n1[1] * n2[0];
-  const double dd = d[0] * d[0] + d[1] * d[1] + d[2] * d[2];
-  const double nn = (n1[0] * n1[0] + n1[1] * n1[1] + n1[2] * n1[2]) * (n2[0] * n2[0] + n2[1] * n2[1] + n2[2] * n2[2]);
+  d[0] = det2(n1[1], n2[2], n1[2], n2[1]);
+  d[1] = det2(n1[2], n2[0], n1[0], n2[2]);
+  d[2] = det2(n1[0], n2[1], n1[1], n2[0]);
+  const double dd = dot3(d[0], d[1], d[2], d[0], d[1], d[2]);
+  const double nn = dot3(n1[0], n1[1], n1[2], n1[0], n1[1], n1[2]) * dot3(n2[0], n2[1], n2[2], n2[0], n2[1], n2[2]);
   if (!(dd > 1e-24 * nn)) return false;
   // x0 = (-w1 (n2 x d) - w2 (d x n1)) / |d|^2
-  const double a0 = n2[1] * d[2] - n2[2] * d[1], a1 = n2[2] * d[0] - n2[0] * d[2], a2 = n2[0] * d[1] - n2[1] * d[0];
-  const double b0 = d[1] * n1[2] - d[2] * n1[1], b1 = d[2] * n1[0] - d[0] * n1[2], b2 = d[0] * n1[1] - d[1] * n1[0];
-  const double inv = 1.0 / dd;
-  x0[0] = (-n1[3] * a0 - n2[3] * b0) * inv;
-  x0[1] = (-n1[3] * a1 - n2[3] * b1) * inv;
-  x0[2] = (-n1[3] * a2 - n2[3] * b2) * inv;
+  const double a0 = det2(n2[1], d[2], n2[2], d[1]), a1 = det2(n2[2], d[0], n2[0], d[2]), a2 = det2(n2[0], d[1], n2[1], d[0]);
+  const double b0 = det2(d[1], n1[2], d[2], n1[1]), b1 = det2(d[2], n1[0], d[0], n1[2]), b2 = det2(d[0], n1[1], d[1], n1[0]);
+  const double inv = __drcp_rn(dd);
+  x0[0] = __fma_rn(-n1[3], a0, -__dmul_rn(n2[3], b0)) * inv;
+  x0[1] = __fma_rn(-n1[3], a1, -__dmul_rn(n2[3], b1)) * inv;
+  x0[2] = __fma_rn(-n1[3], a2, -__dmul_rn(n2[3], b2)) * inv;
   return true;
 }
 
-// Parameter range of the line x0 + s d inside plane n.
-__device__ __forceinline__ void clip_line(const double *n, const double x0[3], const double d[3], double &lo, double &hi) {
-  const double v0 = pval(n, x0[0], x0[1], x0[2]);
-  const double sl = n[0] * d[0] + n[1] * d[1] + n[2] * d[2];
-  if (sl > 0.0) lo = fmax(lo, -v0 / sl);
-  else if (sl < 0.0) hi = fmin(hi, -v0 / sl);
-  else if (v0 < 0.0) hi = -1e300;
-}
-
-// Face f's facet: its edges inside the cone, and the cone planes' lines
-// inside the face (bounded by the face's edge planes and the other cone
-// planes), as boundary segments (U, V) of the facet; emit(c, U, V) for each,
-// c the face's first vertex.
-template <class Emit>
-__device__ __forceinline__ void face_segments(const ConePiece &q, const WarpCell &w, const double *px,
-                                              const double *py, const double *pz, int f, Emit emit) {
-  const int f0 = w.fstart[f], k = w.fstart[f + 1] - f0;
-  const int v0 = w.fv[f0];
-  const double c[3] = {px[v0], py[v0], pz[v0]};
-  for (int i = 0; i < k; ++i) {
-    const int iu = w.fv[f0 + i], iv = w.fv[f0 + (i + 1 == k ? 0 : i + 1)];
-    const double u[3] = {px[iu], py[iu], pz[iu]}, v[3] = {px[iv], py[iv], pz[iv]};
-    double lo = 0.0, hi = 1.0;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) clip_seg(pval(q.c[j], u[0], u[1], u[2]), pval(q.c[j], v[0], v[1], v[2]), lo, hi);
-    if (lo < hi) {
-      const double U[3] = {fma(lo, v[0] - u[0], u[0]), fma(lo, v[1] - u[1], u[1]), fma(lo, v[2] - u[2], u[2])};
-      const double V[3] = {fma(hi, v[0] - u[0], u[0]), fma(hi, v[1] - u[1], u[1]), fma(hi, v[2] - u[2], u[2])};
-      emit(c, U, V);
-    }
-  }
-  const Plane pf = w.plane[f];
-  const double nf[4] = {pf.x, pf.y, pf.z, pf.w};
-#pragma unroll 1
-  for (int j = 0; j < 4; ++j) {
-    double x0[3], d[3];
-    if (!plane_line(nf, q.c[j], x0, d)) continue;
-    double lo = -1e300, hi = 1e300;
-#pragma unroll
-    for (int jj = 0; jj < 4; ++jj)
-      if (jj != j) clip_line(q.c[jj], x0, d, lo, hi);
-    const unsigned char *nb = face_nb(w);
-    for (int i = 0; i < k && lo < hi; ++i) {
-      // the plane of the face's edge (i, i+1)
-      const unsigned e = nb[f0 + i];
-      if (e == 0xffu) continue;
-      const Plane pe = w.plane[e];
-      const double ne[4] = {pe.x, pe.y, pe.z, pe.w};
-      clip_line(ne, x0, d, lo, hi);
-    }
-    if (lo < hi) {
-      const double U[3] = {fma(lo, d[0], x0[0]), fma(lo, d[1], x0[1]), fma(lo, d[2], x0[2])};
-      const double V[3] = {fma(hi, d[0], x0[0]), fma(hi, d[1], x0[1]), fma(hi, d[2], x0[2])};
-      emit(c, U, V);
+// The part [lo, hi] of x0 + s d that sp leaves, as a boundary segment of a
+// facet with point c: its signed tetrahedron (a, c, U, V) into acc (6 * volume
+// * 4 and 6 * volume * 4 * centroid), and with a normal (the facet's plane,
+// Hessian) its triangle (c, U, V) against the outward normal into term.
+template <bool HESS>
+__device__ __noinline__ void add_segment(const Span &sp, const double x0[3], const double d[3], const double c[3],
+                                         const double a[3], double acc[4], const Plane *face, double term[4]) {
+  const double lo = __ddiv_rn(sp.ln, sp.ld), hi = __ddiv_rn(sp.hn, sp.hd);
+  if (!(lo < hi)) return;
+  const double U[3] = {__fma_rn(lo, d[0], x0[0]), __fma_rn(lo, d[1], x0[1]), __fma_rn(lo, d[2], x0[2])};
+  const double V[3] = {__fma_rn(hi, d[0], x0[0]), __fma_rn(hi, d[1], x0[1]), __fma_rn(hi, d[2], x0[2])};
+  const double cx = c[0] - a[0], cy = c[1] - a[1], cz = c[2] - a[2];
+  const double ux = U[0] - a[0], uy = U[1] - a[1], uz = U[2] - a[2];
+  const double vx = V[0] - a[0], vy = V[1] - a[1], vz = V[2] - a[2];
+  const double det = dot3(cx, cy, cz, det2(uy, vz, uz, vy), det2(uz, vx, ux, vz), det2(ux, vy, uy, vx));
+  acc[0] = __fma_rn(det, a[0] + c[0] + U[0] + V[0], acc[0]);
+  acc[1] = __fma_rn(det, a[1] + c[1] + U[1] + V[1], acc[1]);
+  acc[2] = __fma_rn(det, a[2] + c[2] + U[2] + V[2], acc[2]);
+  acc[3] = __fma_rn(det, 4.0, acc[3]);
+  if constexpr (HESS) {
+    if (face) {
+      const double ex = U[0] - c[0], ey = U[1] - c[1], ez = U[2] - c[2];
+      const double fx = V[0] - c[0], fy = V[1] - c[1], fz = V[2] - c[2];
+      const double t = -0.5 * dot3(face->x, face->y, face->z, det2(ey, fz, ez, fy), det2(ez, fx, ex, fz),
+                                   det2(ex, fy, ey, fx));
+      term[0] = t * (c[0] + U[0] + V[0]) * (1.0 / 3.0);
+      term[1] = t * (c[1] + U[1] + V[1]) * (1.0 / 3.0);
+      term[2] = t * (c[2] + U[2] + V[2]) * (1.0 / 3.0);
+      term[3] = t;
     }
   }
 }
 
-__device__ void face_facet(ConePiece &q, const WarpCell &w, const double *px, const double *py, const double *pz,
-                           int f) {
-  face_segments(q, w, px, py, pz, f,
-                [&](const double *c, const double *U, const double *V) { edge_tet(q, c, U, V); });
-}
-
-// The facet of face f inside the cone as Hessian terms: its area (the
-// boundary segments fanned from c, against the face's outward normal -n),
-// and with 4 components its area times its centroid (local frame).
-__device__ __noinline__ void face_piece(const ConePiece &q, const WarpCell &w, const double *px, const double *py,
-                                        const double *pz, int f, double out[4]) {
-  const Plane pf = w.plane[f];
-  double a = 0, mx = 0, my = 0, mz = 0;
-  face_segments(q, w, px, py, pz, f, [&](const double *c, const double *U, const double *V) {
-    const double ux = U[0] - c[0], uy = U[1] - c[1], uz = U[2] - c[2];
-    const double vx = V[0] - c[0], vy = V[1] - c[1], vz = V[2] - c[2];
-    const double t = -0.5 * ((uy * vz - uz * vy) * pf.x + (uz * vx - ux * vz) * pf.y + (ux * vy - uy * vx) * pf.z);
-    a += t;
-    mx += t * (c[0] + U[0] + V[0]) * (1.0 / 3.0);
-    my += t * (c[1] + U[1] + V[1]) * (1.0 / 3.0);
-    mz += t * (c[2] + U[2] + V[2]) * (1.0 / 3.0);
-  });
-  if (w.hc == 1) {
-    out[0] = a;
-  } else {
-    out[0] = mx;
-    out[1] = my;
-    out[2] = mz;
-    out[3] = a;
-  }
-}
-
-// One round of facet pieces (lane: face f >= 0 or none) into w.harea,
-// signed: each lane stages its piece, then lane c adds component c of
-// every staged piece in lane order.
-__device__ __noinline__ void hess_pieces(const ConePiece &q, const WarpCell &w, const double *px, const double *py,
-                                         const double *pz, int f, double sgn, int lane) {
+// One round of facet terms (lane: face f >= 0 or none) into w.harea, signed:
+// each lane stages its term, then lane c adds component c of all of them in
+// lane order.
+__device__ __noinline__ void hess_terms(const WarpCell &w, int f, const double term[4], double sgn, int lane) {
   const int hc = w.hc;
-  double out[4] = {0, 0, 0, 0};
-  if (f >= 0) face_piece(q, w, px, py, pz, f, out);
-  for (int c = 0; c < hc; ++c) w.hstage[lane * hc + c] = sgn * out[c];
+  if (hc == 1) {
+    w.hstage[lane] = sgn * term[3];
+  } else {
+    for (int c = 0; c < 4; ++c) w.hstage[lane * 4 + c] = sgn * term[c];
+  }
   w.hstage_f[lane] = f;
   __syncwarp();
   if (lane < hc)
@@ -1802,216 +1732,288 @@ __device__ __noinline__ void hess_pieces(const ConePiece &q, const WarpCell &w, 
 }
 
 // Sets up the cone of triangle tri from apex a; false for a flat cone.
-__device__ bool cone_setup(ConePiece &q, const DevGrid &g, float4 s, int tri, const double a[3], double &sgn) {
-  const float4 q1 = __ldg(&g.points[__ldg(&g.tris[3 * tri])]);
-  const float4 q2 = __ldg(&g.points[__ldg(&g.tris[3 * tri + 1])]);
-  const float4 q3 = __ldg(&g.points[__ldg(&g.tris[3 * tri + 2])]);
-  const float4 qs[3] = {q1, q2, q3};
-  double d[3][3];
-#pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    q.t[i][0] = double(qs[i].x) - s.x;
-    q.t[i][1] = double(qs[i].y) - s.y;
-    q.t[i][2] = double(qs[i].z) - s.z;
-#pragma unroll
-    for (int k = 0; k < 3; ++k) d[i][k] = q.t[i][k] - a[k];
-  }
-#pragma unroll
-  for (int k = 0; k < 3; ++k) q.a[k] = a[k];
-  const double det = d[0][0] * (d[1][1] * d[2][2] - d[1][2] * d[2][1]) -
-                     d[0][1] * (d[1][0] * d[2][2] - d[1][2] * d[2][0]) +
-                     d[0][2] * (d[1][0] * d[2][1] - d[1][1] * d[2][0]);
+// Every lane of the octet computes the corners, lanes 0..3 a plane each.
+__device__ __forceinline__ bool cone_setup(ConeOct &q, const DevGrid &g, float4 s, int tri, const double a[3],
+                                           double &sgn, int l8) {
+  const float4 q0 = __ldg(&g.points[__ldg(&g.tris[3 * tri])]);
+  float4 q1 = __ldg(&g.points[__ldg(&g.tris[3 * tri + 1])]);
+  float4 q2 = __ldg(&g.points[__ldg(&g.tris[3 * tri + 2])]);
+  double t0[3] = {double(q0.x) - s.x, double(q0.y) - s.y, double(q0.z) - s.z};
+  double t1[3] = {double(q1.x) - s.x, double(q1.y) - s.y, double(q1.z) - s.z};
+  double t2[3] = {double(q2.x) - s.x, double(q2.y) - s.y, double(q2.z) - s.z};
+  const double det =
+      dot3(t0[0] - a[0], t0[1] - a[1], t0[2] - a[2],
+           det2(t1[1] - a[1], t2[2] - a[2], t1[2] - a[2], t2[1] - a[1]),
+           det2(t1[2] - a[2], t2[0] - a[0], t1[0] - a[0], t2[2] - a[2]),
+           det2(t1[0] - a[0], t2[1] - a[1], t1[1] - a[1], t2[0] - a[0]));
   if (!(fabs(det) > 0.0)) return false;
   // the reference's sign: + when the triangle is seen positively from a
   sgn = det > 0.0 ? 1.0 : -1.0;
   if (det < 0.0) {
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-      double x = q.t[1][k];
-      q.t[1][k] = q.t[2][k];
-      q.t[2][k] = x;
-      x = d[1][k];
-      d[1][k] = d[2][k];
-      d[2][k] = x;
+      const double x = t1[k];
+      t1[k] = t2[k];
+      t2[k] = x;
     }
   }
+  if (l8 < 4) {
+    // plane l8 < 3: through a and corners l8, l8 + 1; 3: the triangle's
+    double u[3], v[3], o[3];
 #pragma unroll
-  for (int j = 0; j < 3; ++j) {
-    const double *u = d[j], *v = d[(j + 1) % 3];
-    q.c[j][0] = u[1] * v[2] - u[2] * v[1];
-    q.c[j][1] = u[2] * v[0] - u[0] * v[2];
-    q.c[j][2] = u[0] * v[1] - u[1] * v[0];
-    q.c[j][3] = -(q.c[j][0] * a[0] + q.c[j][1] * a[1] + q.c[j][2] * a[2]);
+    for (int k = 0; k < 3; ++k) {
+      const double p = l8 == 3 ? t1[k] : (l8 == 0 ? t0[k] : (l8 == 1 ? t1[k] : t2[k]));
+      const double r = l8 == 3 ? t2[k] : (l8 == 0 ? t1[k] : (l8 == 1 ? t2[k] : t0[k]));
+      o[k] = l8 == 3 ? t0[k] : a[k];
+      u[k] = p - o[k];
+      v[k] = r - o[k];
+    }
+    const double nx = det2(u[1], v[2], u[2], v[1]), ny = det2(u[2], v[0], u[0], v[2]), nz = det2(u[0], v[1], u[1], v[0]);
+    q.c[l8][0] = nx;
+    q.c[l8][1] = ny;
+    q.c[l8][2] = nz;
+    q.c[l8][3] = -dot3(nx, ny, nz, o[0], o[1], o[2]);
   }
-  const double e1[3] = {q.t[1][0] - q.t[0][0], q.t[1][1] - q.t[0][1], q.t[1][2] - q.t[0][2]};
-  const double e2[3] = {q.t[2][0] - q.t[0][0], q.t[2][1] - q.t[0][1], q.t[2][2] - q.t[0][2]};
-  q.c[3][0] = e1[1] * e2[2] - e1[2] * e2[1];
-  q.c[3][1] = e1[2] * e2[0] - e1[0] * e2[2];
-  q.c[3][2] = e1[0] * e2[1] - e1[1] * e2[0];
-  q.c[3][3] = -(q.c[3][0] * q.t[0][0] + q.c[3][1] * q.t[0][1] + q.c[3][2] * q.t[0][2]);
-  q.acc[0] = q.acc[1] = q.acc[2] = q.acc[3] = 0.0;
+  if (l8 == 4)
+    for (int k = 0; k < 3; ++k) {
+      q.t[0][k] = t0[k];
+      q.t[1][k] = t1[k];
+      q.t[2][k] = t2[k];
+    }
   return true;
 }
 
-// Cone pieces of triangles tids[t0, t1) (at most 32), one per lane, summed
-// over the warp into acc.  Needs build_faces.
+// Cone pieces of triangles tids[t0, t1), summed into acc.  Needs
+// build_faces.  Octet o takes triangles t0 + o, t0 + 4 + o, ...
 template <bool HESS = false>
 __device__ void facet_triangles(const WarpCell &w, const double *px, const double *py, const double *pz,
                                 const DevGrid &g, float4 s, const int *tids, int t0, int t1, const double a[3],
                                 double acc[4], int lane, unsigned long long *ctr) {
-  ConePiece q;
-  double sgn = 0.0;
-  const bool act = t0 + lane < t1 && cone_setup(q, g, s, tids[t0 + lane], a, sgn);
-  if (!act) q.acc[0] = q.acc[1] = q.acc[2] = q.acc[3] = 0.0;
-  const int np = w.np;
-  // t ∩ C, seen from a (outer side): edges t0 -> t2 -> t1 -> t0 clipped by
-  // the cell planes, and the lines of the cell planes that cut t
-  // cone axis and half-angle seen from a (floats, for culling the faces)
-  float tux = 0.f, tuy = 0.f, tuz = 0.f, tth = 4.f, tc = -1.f, ts = 0.f;
-  if (act) {
+  const int np = w.np, nv = w.nv, l8 = lane & 7, oct = lane >> 3;
+  const unsigned osh = lane & 24, lt8 = (1u << l8) - 1u;
+  auto bits = [&](bool p) { return (__ballot_sync(kFull, p) >> osh) & 0xffu; };
+  // the octet's work space
+  const unsigned co = align16(unsigned(sizeof(ConeOct)) + nv + np);
+  unsigned char *base = reinterpret_cast<unsigned char *>(w.cx) + oct * co;
+  ConeOct &q = *reinterpret_cast<ConeOct *>(base);
+  unsigned char *vm = base + sizeof(ConeOct);  // per vertex: bit j, inside cone plane j
+  unsigned char *cutp = vm + nv;               // the cell planes that cut the triangle
+  unsigned *tasks = reinterpret_cast<unsigned *>(w.bcw);
+  const unsigned char *nb = face_nb(w);
+  double sum[4] = {0, 0, 0, 0};
+#pragma unroll 1
+  for (int b0 = t0; b0 < t1; b0 += 4) {
+    double sgn = 0.0;
+    double part[4] = {0, 0, 0, 0};
+    double term[4] = {0, 0, 0, 0};
+    bool act = b0 + oct < t1;
+    __syncwarp();
+    if (act) act = cone_setup(q, g, s, tids[b0 + oct], a, sgn, l8);
+    __syncwarp();
+    // the cell's vertices against the cone's planes
+#pragma unroll 1
+    for (int v = l8; v < nv && act; v += 8) {
+      const double x = px[v], y = py[v], z = pz[v];
+      unsigned m = 0;
 #pragma unroll
-    for (int i = 0; i < 3; ++i) {
-      const float dx = float(q.t[i][0] - a[0]), dy = float(q.t[i][1] - a[1]), dz = float(q.t[i][2] - a[2]);
-      const float il = rsqrtf(fmaxf(dx * dx + dy * dy + dz * dz, 1e-30f));
-      tux += dx * il;
-      tuy += dy * il;
-      tuz += dz * il;
+      for (int j = 0; j < 4; ++j) m |= (pval(q.c[j], x, y, z) >= 0.0 ? 1u : 0u) << j;
+      vm[v] = (unsigned char)m;
     }
-    const float ul = rsqrtf(fmaxf(tux * tux + tuy * tuy + tuz * tuz, 1e-30f));
-    tux *= ul;
-    tuy *= ul;
-    tuz *= ul;
-    float cmin = 1.f;
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-      const float dx = float(q.t[i][0] - a[0]), dy = float(q.t[i][1] - a[1]), dz = float(q.t[i][2] - a[2]);
-      const float il = rsqrtf(fmaxf(dx * dx + dy * dy + dz * dz, 1e-30f));
-      cmin = fminf(cmin, (dx * tux + dy * tuy + dz * tuz) * il);
-    }
-    tth = acosf(fmaxf(-1.f, fminf(1.f, cmin)));
-    tc = cosf(tth);
-    ts = sinf(tth);
-  }
-  if (act) {
-    // bounding sphere of t: a plane farther than its radius does not cut t
-    const double gx = (q.t[0][0] + q.t[1][0] + q.t[2][0]) * (1.0 / 3.0);
-    const double gy = (q.t[0][1] + q.t[1][1] + q.t[2][1]) * (1.0 / 3.0);
-    const double gz = (q.t[0][2] + q.t[1][2] + q.t[2][2]) * (1.0 / 3.0);
-    double r2 = 0.0;
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-      const double dx = q.t[i][0] - gx, dy = q.t[i][1] - gy, dz = q.t[i][2] - gz;
-      r2 = fmax(r2, dx * dx + dy * dy + dz * dz);
-    }
-    const double rad = sqrt(r2) * (1.0 + 1e-9) + 1e-9;
-    double lo[3] = {0.0, 0.0, 0.0}, hi[3] = {1.0, 1.0, 1.0};
-    for (int kb = 0; kb < np; kb += 64) {
-      unsigned long long cutm = 0;
-      const int ke = min(np, kb + 64);
-      for (int kp = kb; kp < ke; ++kp) {
-        const Plane pl = w.plane[kp];
+    // the planes of the cell that cut t; t ∩ C is empty when one holds none of it
+    int ncut = 0;
+    bool none = false;
+#pragma unroll 1
+    for (int k0 = 0; k0 < np; k0 += 8) {
+      const int k = k0 + l8;
+      int out = 0;
+      if (act && k < np) {
+        const Plane pl = w.plane[k];
         const double n[4] = {pl.x, pl.y, pl.z, pl.w};
-        if (pval(n, gx, gy, gz) > rad) continue;
-        const double e0 = pval(n, q.t[0][0], q.t[0][1], q.t[0][2]);
-        const double e1 = pval(n, q.t[1][0], q.t[1][1], q.t[1][2]);
-        const double e2 = pval(n, q.t[2][0], q.t[2][1], q.t[2][2]);
-        if (e0 >= 0.0 && e1 >= 0.0 && e2 >= 0.0) continue;
-        cutm |= 1ull << (kp - kb);
-        clip_seg(e0, e2, lo[0], hi[0]);
-        clip_seg(e2, e1, lo[1], hi[1]);
-        clip_seg(e1, e0, lo[2], hi[2]);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) out += pval(n, q.t[i][0], q.t[i][1], q.t[i][2]) < 0.0 ? 1 : 0;
       }
-      // lines of the cutting planes in the triangle's plane (direction
-      // n_3 x n_k keeps t ∩ C on the left seen from a), bounded by t's edges
-      // and the other cutting planes: every other plane holds all of t
-      const unsigned long long all = cutm;
-      while (cutm) {
-        const int kp = kb + __ffsll(cutm) - 1;
-        cutm &= cutm - 1;
-        const Plane pl = w.plane[kp];
+      const unsigned m = bits(out > 0);
+      none |= bits(out == 3) != 0;
+      if (out > 0) cutp[ncut + __popc(m & lt8)] = (unsigned char)k;
+      ncut += __popc(m);
+    }
+    __syncwarp();
+    if (none || !act) ncut = -1;
+    // t ∩ C, seen from a (outer side): the edges t0 -> t2 -> t1 -> t0 (tasks 0
+    // .. 2) inside the cutting planes, and the lines of the cutting planes in
+    // the triangle's plane (direction n_3 x n_k keeps t ∩ C on the left seen
+    // from a) inside t's edges and the other cutting planes
+#pragma unroll 1
+    for (int k0 = 0; __any_sync(kFull, k0 < ncut + 3 && ncut >= 0); k0 += 8) {
+      const int k = k0 + l8;
+      if (ncut < 0 || k >= ncut + 3) continue;
+      double x0[3], d[3];
+      Span sp{0.0, 1.0, 1.0, 1.0};
+      bool ok = true;
+      if (k < 3) {
+        const double *u = q.t[k == 0 ? 0 : 3 - k], *v = q.t[k == 2 ? 0 : 2 - k];
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+          x0[i] = u[i];
+          d[i] = v[i] - u[i];
+        }
+      } else {
+        const Plane pl = w.plane[cutp[k - 3]];
         const double n[4] = {pl.x, pl.y, pl.z, pl.w};
-        double x0[3], d[3];
-        if (!plane_line(q.c[3], n, x0, d)) continue;
-        double l = -1e300, h = 1e300;
-#pragma unroll
-        for (int j = 0; j < 3; ++j) clip_line(q.c[j], x0, d, l, h);
-        unsigned long long others = all & ~(1ull << (kp - kb));
-        while (others && l < h) {
-          const int k2 = kb + __ffsll(others) - 1;
-          others &= others - 1;
-          const Plane p2 = w.plane[k2];
-          const double n2[4] = {p2.x, p2.y, p2.z, p2.w};
-          clip_line(n2, x0, d, l, h);
-        }
-        // cutting planes of the other batches
-        for (int k2 = 0; k2 < np && l < h && np > 64; ++k2) {
-          if (k2 >= kb && k2 < ke) continue;
-          const Plane p2 = w.plane[k2];
-          const double n2[4] = {p2.x, p2.y, p2.z, p2.w};
-          clip_line(n2, x0, d, l, h);
-        }
-        if (l < h) {
-          const double U[3] = {fma(l, d[0], x0[0]), fma(l, d[1], x0[1]), fma(l, d[2], x0[2])};
-          const double V[3] = {fma(h, d[0], x0[0]), fma(h, d[1], x0[1]), fma(h, d[2], x0[2])};
-          edge_tet(q, q.t[0], U, V);
-        }
+        ok = plane_line(q.c[3], n, x0, d);
+        sp = Span{-1e200, 1.0, 1e200, 1.0};
       }
+#pragma unroll 1
+      for (int i = 0; i < ncut + 3; ++i) {
+        if (i == k || (i < 3 && k < 3)) continue;
+        const double *n = i < 3 ? q.c[i] : reinterpret_cast<const double *>(&w.plane[cutp[i - 3]]);
+        sp.clip_line(n, x0, d);
+      }
+      if (ok && sp.open()) add_segment<false>(sp, x0, d, q.t[0], a, part, nullptr, term);
     }
-    const int ord[4] = {0, 2, 1, 0};
+    // the faces that the cone may meet (a vertex inside each of its planes),
+    // eight at a time; their edges not beyond one plane, and the lines of the
+    // cone planes that cut them, go to the warp's list of tasks, one per lane
+    // when run
+    for (int i = 0; i < 4; ++i) {
+      sum[i] = __fma_rn(sgn, part[i], sum[i]);
+      part[i] = 0.0;
+    }
+    int nt = 0;        // tasks listed
+    int f0 = 0;        // the next group of faces
+    int it = 0, its = 0;  // the group's next append of eight: edges, then lines of plane 0 .. 3
+    int fs = 0, k = 0, ke = 0, face = -1, te = 0;  // the lane's face: its list, edges before the next face, all edges
+    unsigned lines = 0;
+#pragma unroll 1
+    for (;;) {
+      const bool end = it >= its && f0 >= np;
+      if (__all_sync(kFull, end) || nt > kConeTasks - 32) {
+        __syncwarp();
+#pragma unroll 1
+        for (int r0 = 0; r0 < nt; r0 += 32) {
+          int ff = -1, o = 0;
+          double part2[4] = {0, 0, 0, 0};
+          if (r0 + lane < nt) {
+            const unsigned e = tasks[r0 + lane];
+            o = int(e >> 24);
+            ff = int((e >> 16) & 0xffu);
+            const unsigned char *ob = reinterpret_cast<const unsigned char *>(w.cx) + o * co;
+            const ConeOct &qo = *reinterpret_cast<const ConeOct *>(ob);
+            const unsigned char *vmo = ob + sizeof(ConeOct);
+            const int s0 = w.fstart[ff], kk = w.fstart[ff + 1] - s0, ic = w.fv[s0], i = int(e & 0x7fffu);
+            double x0[3], d[3];
+            Span sp{0.0, 1.0, 1.0, 1.0};
+            bool ok = true;
+            int last = 4, skip = -1;  // the planes that clip it: 4 of the cone, the face's edge planes
+            if (e & 0x8000u) {
+              const double *nf = reinterpret_cast<const double *>(&w.plane[ff]);
+              ok = plane_line(nf, qo.c[i], x0, d);
+              sp = Span{-1e200, 1.0, 1e200, 1.0};
+              last = 4 + kk;
+              skip = i;
+            } else {
+              const int iu = w.fv[s0 + i], iv = w.fv[s0 + (i + 1 == kk ? 0 : i + 1)];
+              x0[0] = px[iu];
+              x0[1] = py[iu];
+              x0[2] = pz[iu];
+              d[0] = px[iv] - x0[0];
+              d[1] = py[iv] - x0[1];
+              d[2] = pz[iv] - x0[2];
+              if ((vmo[iu] & vmo[iv]) == 15u) last = 0;  // the whole edge
+            }
+#pragma unroll 1
+            for (int m = 0; m < last; ++m) {
+              if (m == skip) continue;
+              const double *n = qo.c[m & 3];
+              if (m >= 4) {
+                const unsigned e2 = nb[s0 + m - 4];
+                if (e2 == 0xffu) continue;
+                n = reinterpret_cast<const double *>(&w.plane[e2]);
+              }
+              sp.clip_line(n, x0, d);
+            }
+            if (HESS) term[0] = term[1] = term[2] = term[3] = 0.0;
+            const double c[3] = {px[ic], py[ic], pz[ic]};
+            if (ok && sp.open()) add_segment<HESS>(sp, x0, d, c, a, part2, &w.plane[ff], term);
+          }
+          const double so = __shfl_sync(kFull, sgn, o * 8);
 #pragma unroll
-    for (int i = 0; i < 3; ++i) {
-      if (!(lo[i] < hi[i])) continue;
-      const double *u = q.t[ord[i]], *v = q.t[ord[i + 1]];
-      const double U[3] = {fma(lo[i], v[0] - u[0], u[0]), fma(lo[i], v[1] - u[1], u[1]), fma(lo[i], v[2] - u[2], u[2])};
-      const double V[3] = {fma(hi[i], v[0] - u[0], u[0]), fma(hi[i], v[1] - u[1], u[1]), fma(hi[i], v[2] - u[2], u[2])};
-      edge_tet(q, q.t[0], U, V);
-    }
-  }
-  // faces of the cell that the cone meets beyond t, 64 at a time
-  for (int fb = 0; fb < np; fb += kFaceCap) {
-    unsigned long long hit = 0;
-    if (act) {
-      const int fe = min(np, fb + kFaceCap);
-      const float *ang = face_angles(w);
-      const int acap = face_angle_cap(w);
-      for (int f = fb; f < fe; ++f) {
-        const int f0 = w.fstart[f], k = w.fstart[f + 1] - f0;
-        if (k < 3) continue;
-        if (f < acap) {
-          // the cones from a around the face and around t must meet (both
-          // narrower than a half-space, so each holds its convex hull)
-          const float *g4 = ang + 6 * f;
-          if (g4[3] < 1.5f && tth < 1.5f) {
-            const float cosang = g4[0] * tux + g4[1] * tuy + g4[2] * tuz;
-            if (cosang < g4[4] * tc - g4[5] * ts - 1e-3f) continue;
+          for (int i = 0; i < 4; ++i) sum[i] = __fma_rn(so, part2[i], sum[i]);
+          if constexpr (HESS) {
+            if (w.harea) hess_terms(w, ff, term, so, lane);
           }
         }
-        unsigned any_in = 0;
-        for (int i = 0; i < k && any_in != 15u; ++i) {
-          const int v = w.fv[f0 + i];
-          const double x = px[v], y = py[v], z = pz[v];
-#pragma unroll
-          for (int j = 0; j < 4; ++j) any_in |= (pval(q.c[j], x, y, z) >= 0.0 ? 1u : 0u) << j;
+        __syncwarp();
+        nt = 0;
+        if (__all_sync(kFull, end)) break;
+      }
+      if (it >= its) {
+        // the next eight faces, one per lane
+        face = f0 + l8;
+        f0 += 8;
+        k = 0;
+        lines = 0;
+        bool hit = false;
+        if (act && face < np) {
+          fs = w.fstart[face];
+          k = w.fstart[face + 1] - fs;
+          unsigned any = 0, all = 15u;
+#pragma unroll 1
+          for (int i = 0; i < k; ++i) {
+            const unsigned m = vm[w.fv[fs + i]];
+            any |= m;
+            all &= m;
+          }
+          hit = k >= 3 && any == 15u;
+          if (hit) lines = ~all & 15u;
         }
-        if (any_in == 15u) hit |= 1ull << (f - fb);
-      }
-    }
-    while (__any_sync(kFull, hit != 0)) {
-      int f = -1;
-      if (hit) {
-        f = fb + __ffsll(hit) - 1;
-        hit &= hit - 1;
-        face_facet(q, w, px, py, pz, f);
-      }
-      if constexpr (HESS) {
-        if (w.harea) hess_pieces(q, w, px, py, pz, f, sgn, lane);
+        if (!hit) k = 0;
+        ke = k;
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) {
+          const int x = __shfl_up_sync(kFull, ke, o, 8);
+          if (l8 >= o) ke += x;
+        }
+        te = __shfl_sync(kFull, ke, 7, 8);
+        const int ee = (__reduce_max_sync(kFull, te) + 7) / 8;
+        it = 0;
+        its = ee > 0 ? ee + 4 : 0;
+      } else {
+        bool want = false;
+        unsigned entry = 0;
+        if (it + 4 < its) {
+          // the group's edge number 8 it + l8: of the first face whose end
+          // lies past it
+          const int e = 8 * it + l8;
+          int owner = 0;
+#pragma unroll
+          for (int step = 4; step > 0; step >>= 1) {
+            const int x = __shfl_sync(kFull, ke, owner + step - 1, 8);
+            if (x <= e) owner += step;
+          }
+          const int end_e = __shfl_sync(kFull, ke, owner, 8), kk = __shfl_sync(kFull, k, owner, 8),
+                    s0 = __shfl_sync(kFull, fs, owner, 8);
+          if (e < te) {
+            const int i = e - (end_e - kk);
+            want = (vm[w.fv[s0 + i]] | vm[w.fv[s0 + (i + 1 == kk ? 0 : i + 1)]]) == 15u;
+            entry = unsigned(f0 - 8 + owner) << 16 | unsigned(i);
+          }
+        } else {
+          const int j = it + 4 - its;
+          want = (lines >> j) & 1u;
+          entry = unsigned(face) << 16 | 0x8000u | unsigned(j);
+        }
+        const unsigned m = __ballot_sync(kFull, want);
+        if (want) tasks[nt + __popc(m & lanemask_lt(lane))] = unsigned(oct) << 24 | entry;
+        nt += __popc(m);
+        ++it;
       }
     }
   }
   count(ctr, kCtrExports, t1 - t0, lane);
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
-    double v = act ? sgn * q.acc[k] * (1.0 / 24.0) : 0.0;
+    double v = sum[k] * (1.0 / 24.0);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
     acc[k] += v;
@@ -2069,13 +2071,32 @@ __device__ void park_cell(const WarpCell &w, const DeferQueue &dq, int slot, con
   cb = __shfl_sync(kFull, cb, 0);
   for (int c = lane; c < nch; c += 32) dq.chunk_slot[cb + c] = slot;
   for (int i = lane; i < w.np; i += 32) pl[i] = w.plane[i];
-  for (int v = lane; v < w.nv; v += 32) {
-    vx[v] = w.cx[v];
-    vy[v] = w.cy[v];
-    vz[v] = w.cz[v];
-    vw[v] = w.cw[v];
-    vd[v] = w.d2[v];
-    vt[v] = w.tri[v];
+  if (inner) {
+    // the cone kernel needs the vertices' positions and the faces: built once
+    // per cell and not per work item
+    build_faces(w, w.bcx, w.bcy, w.bcz, lane);
+    int *fs = reinterpret_cast<int *>(vw);
+    unsigned char *fv = reinterpret_cast<unsigned char *>(fs + L.Pc + 1), *nb = fv + 3 * w.nv;
+    for (int v = lane; v < w.nv; v += 32) {
+      vx[v] = w.bcx[v];
+      vy[v] = w.bcy[v];
+      vz[v] = w.bcz[v];
+      vt[v] = w.tri[v];
+    }
+    for (int i = lane; i <= w.np; i += 32) fs[i] = w.fstart[i];
+    for (int i = lane; i < 3 * w.nv; i += 32) {
+      fv[i] = w.fv[i];
+      nb[i] = face_nb(w)[i];
+    }
+  } else {
+    for (int v = lane; v < w.nv; v += 32) {
+      vx[v] = w.cx[v];
+      vy[v] = w.cy[v];
+      vz[v] = w.cz[v];
+      vw[v] = w.cw[v];
+      vd[v] = w.d2[v];
+      vt[v] = w.tri[v];
+    }
   }
   if (!list_in_place)
     for (int i = lane; i < nuniq; i += 32) tl[i] = w.tlist[i];
@@ -2295,47 +2316,45 @@ __device__ int restrict_to_domain(WarpCell &w, const CellLaunch &a, const Layout
   if (nuniq == 0 && !ahead) return kSuccess;
   if (lane < 3) w.pts[lane] = pt0[lane];
   __syncwarp();
-  if (ahead) {
-    // its slot is taken: parked even without triangles.  Without an inner
-    // apex the cones clip the cell, which depends on the retry pass's P and
-    // V: the retries take it, as a triangle overflow now
-    if (!inner) {
-      park_fixed(dq, slot, a.diag, sid_of_cell, kTriangleOverflow, lane);
-    } else {
-      park_cell(w, dq, slot, L, a.diag, sid_of_cell, nuniq, inner, acc, lane, true);
-      // the retry passes' T schedule follows the counts settled ahead
-      if (lane == 0) atomicMax(a.ahead_max ? a.ahead_max : &dq.counters[3], ntr);
-    }
+  // a cell parked ahead has its slot: parked even without triangles.  Without
+  // an inner apex the cones clip the cell, which depends on the retry pass's
+  // P and V: the retries take it, as a triangle overflow now
+  if (ahead && !inner) {
+    park_fixed(dq, slot, a.diag, sid_of_cell, kTriangleOverflow, lane);
     return kDeferred;
   }
-  if (dq.slots && (!INL || nuniq > dq.inline_max)) {
-    // park the cell: its triangles become work items of k_cone
-    int slot = 0;
+  if (!ahead && dq.slots && (!INL || nuniq > dq.inline_max)) {
     if (lane == 0) slot = atomicAdd(&dq.counters[0], 1);
     slot = __shfl_sync(kFull, slot, 0);
-    if (slot < dq.capacity) {
-      park_cell(w, dq, slot, L, a.diag, sid_of_cell, nuniq, inner, acc, lane);
-      return kDeferred;
-    }
+  } else if (!ahead) {
+    slot = dq.capacity;
+  }
+  if (slot < dq.capacity) {
+    // park the cell: its triangles become work items of k_cone
+    park_cell(w, dq, slot, L, a.diag, sid_of_cell, nuniq, inner, acc, lane, ahead);
+    // the retry passes' T schedule follows the counts settled ahead
+    if (ahead && lane == 0) atomicMax(a.ahead_max ? a.ahead_max : &dq.counters[3], ntr);
+    return kDeferred;
   }
   if constexpr (!INL) {
     return kParkOverflow;  // re-run by the inline variant
   } else {
     if (inner) {
-      build_faces(w, w.bcx, w.bcy, w.bcz, pt0, lane);
-      for (int b0 = 0; b0 < nuniq; b0 += 32)
-        facet_triangles<INL>(w, w.bcx, w.bcy, w.bcz, g, s, w.tlist, b0, min(nuniq, b0 + 32), pt0, acc, lane, ctr);
+      build_faces(w, w.bcx, w.bcy, w.bcz, lane);
+      for (int b0 = 0; b0 < nuniq; b0 += kConeChunk)
+        facet_triangles<INL>(w, w.bcx, w.bcy, w.bcz, g, s, w.tlist, b0, min(nuniq, b0 + kConeChunk), pt0, acc, lane,
+                             ctr);
       return kSuccess;
     }
     const int bk_nv = w.nv, bk_np = w.np;
     backup<VS>(w, lane);
-    // the triangles in chunks of 32, each summed on its own and then added,
+    // the triangles in chunks, each summed on its own and then added,
     // as k_cone sums a parked cell: a cell's result does not depend on
     // whether it was parked
-    for (int c0 = 0; c0 < nuniq; c0 += 32) {
+    for (int c0 = 0; c0 < nuniq; c0 += kConeChunk) {
       double part[4] = {0, 0, 0, 0};
       int fail_at = 0;
-      const int st = cone_triangles<VS, INL>(w, a, s, w.tlist, c0, min(nuniq, c0 + 32), bk_nv, bk_np, inner, part,
+      const int st = cone_triangles<VS, INL>(w, a, s, w.tlist, c0, min(nuniq, c0 + kConeChunk), bk_nv, bk_np, inner, part,
                                         fail_at, lane, ctr, tr, trcap);
       if (st != kSuccess) return st;
       for (int d = 0; d < 4; ++d) acc[d] += part[d];
@@ -3068,20 +3087,27 @@ __device__ __forceinline__ void cone_items(const DeferQueue &dq, const Layout &L
     const CellLaunch &a = desc(h->diag);
     if constexpr (Desc::kBatch) w.vc = vertex_capacity(a, L);
     for (int i = lane; i < np; i += 32) w.plane[i] = pl[i];
-    for (int v = lane; v < nv; v += 32) {
-      w.cx[v] = vx[v];
-      w.cy[v] = vy[v];
-      w.cz[v] = vz[v];
-      w.cw[v] = vw[v];
-      w.d2[v] = vd[v];
-      w.tri[v] = vt[v];
-      if (!inner) {
+    if (inner) {
+      const int *fs = reinterpret_cast<const int *>(vw);
+      const unsigned char *fv = reinterpret_cast<const unsigned char *>(fs + L.Pc + 1), *nb = fv + 3 * nv;
+      for (int v = lane; v < nv; v += 32) {
         w.bcx[v] = vx[v];
         w.bcy[v] = vy[v];
         w.bcz[v] = vz[v];
-        w.bcw[v] = vw[v];
-        w.bd2[v] = vd[v];
-        w.btri[v] = vt[v];
+      }
+      for (int i = lane; i <= np; i += 32) w.fstart[i] = fs[i];
+      for (int i = lane; i < 3 * nv; i += 32) {
+        w.fv[i] = fv[i];
+        face_nb(w)[i] = nb[i];
+      }
+    } else {
+      for (int v = lane; v < nv; v += 32) {
+        w.cx[v] = w.bcx[v] = vx[v];
+        w.cy[v] = w.bcy[v] = vy[v];
+        w.cz[v] = w.bcz[v] = vz[v];
+        w.cw[v] = w.bcw[v] = vw[v];
+        w.d2[v] = w.bd2[v] = vd[v];
+        w.tri[v] = w.btri[v] = vt[v];
       }
     }
     if (lane < 3) w.pts[lane] = h->pt0[lane];
@@ -3094,9 +3120,7 @@ __device__ __forceinline__ void cone_items(const DeferQueue &dq, const Layout &L
     int st;
     if (inner) {
       const double ap[3] = {h->pt0[0], h->pt0[1], h->pt0[2]};
-      build_faces(w, w.bcx, w.bcy, w.bcz, ap, lane);
-      for (int b0 = t0; b0 < t1; b0 += 32)
-        facet_triangles(w, w.bcx, w.bcy, w.bcz, a.grid, s, tl, b0, min(t1, b0 + 32), ap, acc, lane, a.counters);
+      facet_triangles(w, w.bcx, w.bcy, w.bcz, a.grid, s, tl, t0, t1, ap, acc, lane, a.counters);
       st = kSuccess;
     } else {
       st = cone_triangles<VS>(w, a, s, tl, t0, t1, nv, np, false, acc, fail_at, lane, a.counters, nullptr, 0);

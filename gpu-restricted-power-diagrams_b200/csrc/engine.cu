@@ -507,7 +507,7 @@ int run_pass(rpd_solver *s, const int *ids, int num, int K, int P, int V, int T,
     const int t_slot = std::max(T, T_ahead);
     dq.capacity = std::min(num, std::max(32768, s->n / 8));
     dq.slot_bytes = defer_slot_bytes(P, V, t_slot);
-    dq.chunk = 32;  // a warp's lanes take one triangle each
+    dq.chunk = kConeChunk;
     dq.inline_max = 16;
     dq.max_chunks = std::max(1, (t_slot + dq.chunk - 1) / dq.chunk);
     a.T_ahead = T_ahead > T ? T_ahead : 0;
