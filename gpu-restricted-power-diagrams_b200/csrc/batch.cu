@@ -45,7 +45,7 @@ struct DiagStatic {
   int out_domain;  // start-corner fallback of the retry passes
   int early_out, inner_apex;
   const int *wmin;  // the smallest weight of the seeds that are not walls (float_to_ordered)
-  int T_ahead;      // first pass: triangle overflows up to this count parked at once (0: off)
+  int T_ahead;      // triangle overflows up to this count parked at once in the first pass (0: off in every pass)
   int probe;        // 1: the outside probe settles the seeds it can before the first pass
   // --hessian rows (H > 0): per seed H facets of HC values and their
   // neighbours, as rpd_solver_launch writes them (the inline kernels only)
@@ -101,6 +101,7 @@ struct PassArgs {
   long long retry_cap;  // entries of retry_knn
   DeferQueue defer;
   ClipHand hand;
+  int T_slot;          // triangles a parked cell's slot holds
   int Pb, Vb, Tb, Kb;  // caps the pass's launches hold
 };
 
@@ -281,8 +282,9 @@ __global__ void __launch_bounds__(1024) k_plan(const DiagStatic *__restrict__ ds
     a.T = s.T;
     a.cube_eps = g.cube_eps;
     a.out_domain = pa.pass == 0 ? 0 : g.out_domain;
-    if (pa.pass == 0 && pa.defer.slots) {
-      a.T_ahead = g.T_ahead;
+    if (g.T_ahead > 0 && pa.defer.slots) {
+      const int ta = pa.pass == 0 ? g.T_ahead : min(t_ahead_cap(s.P, s.K, s.T, g.max_extra - s.step), pa.T_slot);
+      a.T_ahead = ta > s.T ? ta : 0;
       a.out_domain_ahead = g.out_domain;
       a.ahead_max = &s.ahead_max;
     }
@@ -712,7 +714,11 @@ int capture(rpd_batch *b) {
   const int cap0 = int(std::min<long long>(cells, std::max<long long>(32768, cells / 8)));
   // the first pass's slots hold the triangle overflows parked ahead
   int Tslot0 = Tb[0];
-  for (int d = 0; d < nd; ++d) Tslot0 = std::max(Tslot0, G[d].T_ahead);
+  int Tlater = 0;  // the most a later pass parks ahead
+  for (int d = 0; d < nd; ++d) {
+    Tslot0 = std::max(Tslot0, G[d].T_ahead);
+    if (G[d].T_ahead > 0) Tlater = std::max(Tlater, std::min(grow(G[d].T0, G[d].max_extra), kMaxT));
+  }
   const size_t slot0 = defer_slot_bytes(Pb[0], Vb[0], Tslot0);
   const size_t items0 = size_t(cap0) * std::max(1, (Tslot0 + chunk - 1) / chunk);
   if (any_grid && defer) {
@@ -798,6 +804,7 @@ int capture(rpd_batch *b) {
                                                            b->s0.as<int>());
       }
       PassArgs pa0;
+      pa0.T_slot = 0;
       pa0.pass = 0;
       pa0.final_ = 0;
       pa0.retry_knn = b->retry_knn.as<unsigned>();
@@ -842,6 +849,7 @@ int capture(rpd_batch *b) {
   auto mark = [&](cudaEvent_t ev) { return cudaEventRecordWithFlags(ev, st, cudaEventRecordExternal); };
   for (int j = 0; j < passes; ++j) {
     PassArgs pa;
+    pa.T_slot = 0;
     pa.pass = j;
     pa.final_ = 0;
     pa.retry_knn = b->retry_knn.as<unsigned>();
@@ -852,7 +860,8 @@ int capture(rpd_batch *b) {
     pa.Kb = Kb[j];
     DeferQueue dq;
     if (any_grid && defer) {
-      const int Ts = j == 0 ? Tslot0 : Tb[j];
+      const int Ts = j == 0 ? Tslot0 : std::max(Tb[j], Tlater);
+      pa.T_slot = Ts;
       dq.slot_bytes = defer_slot_bytes(Pb[j], Vb[j], Ts);
       dq.chunk = chunk;
       dq.inline_max = 16;
@@ -910,7 +919,7 @@ int capture(rpd_batch *b) {
     cb.P = Pb[j];
     cb.V = Vb[j];
     cb.T = Tb[j];
-    cb.T_slot = j == 0 && dq.slots ? Tslot0 : 0;
+    cb.T_slot = dq.slots ? pa.T_slot : 0;
     cb.HC = hess_hc;
     cb.disjoint = all_disjoint;
     cb.after_cell = j == 0 ? b->ev[2] : nullptr;

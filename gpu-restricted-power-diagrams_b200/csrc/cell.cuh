@@ -94,8 +94,8 @@ struct CellLaunch {
   // clipping precision: 0 FP64; 1 mixed (FP32 with FP64 escalation, the FP64
   // clipping's decisions); 2 plain FP32 (float planes, no escalation)
   int precision = 0;
-  // first pass: a cell whose clip succeeded and whose range holds more than T
-  // but at most T_ahead triangles (with disjoint lists, counted by grid.tsat)
+  // a cell whose clip succeeded and whose range holds more than T but at most
+  // T_ahead triangles (with disjoint lists, counted by grid.tsat)
   // is parked now with all of them -- the result the retry passes would give
   // it -- its start corner found as they would (out_domain_ahead); 0: off
   int T_ahead = 0;
@@ -153,6 +153,22 @@ constexpr int kTraceRecord = 12;
 constexpr int kMaxP = 255;
 constexpr int kMaxV = 256;
 constexpr int kMaxT = 4096;
+
+// The T of the last retry pass that surely runs after a cell's triangle
+// overflow in a pass of these caps: passes grow T x1.5 while the cell fails,
+// up to max_extra more, and stop once P or K (assumed to grow in every pass)
+// outgrow their limits (voronoi.cpp:867); 0 when no retry surely runs.
+__host__ __device__ inline int t_ahead_cap(int P, int K, int T, int max_extra) {
+  int ahead = 0;
+  for (int j = 0; j < max_extra; ++j) {
+    P = int(P * 1.5);
+    K = int(K * 1.5);
+    if (P > kMaxP || K > 256) break;
+    T = int(T * 1.5) < kMaxT ? int(T * 1.5) : kMaxT;
+    ahead = T;
+  }
+  return ahead;
+}
 
 // Shared memory bytes one warp needs for these caps.
 size_t cell_warp_smem(int P, int V, int T, bool grid);

@@ -2606,7 +2606,7 @@ __device__ __forceinline__ void cell_row(const CellLaunch &a, const Layout &L, u
     if (a.tri_count && a.border_d == 0) {
       if (a.tri_first) {
         if (lane == 0) a.tri_count[sid] = 0;
-      } else if (a.tri_count[sid] > a.T) {
+      } else if (a.tri_count[sid] > max(a.T, a.T_ahead)) {
         // clipped again it would be the same cell, past T again
         if (lane == 0) {
           a.status[sid] = kTriangleOverflow;

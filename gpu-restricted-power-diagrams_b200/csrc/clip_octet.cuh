@@ -448,7 +448,7 @@ __device__ __forceinline__ void clip_octet(const CellLaunch &a, const OctLayout 
     if (GRID && a.tri_count) {
       if (a.tri_first) {
         if (l8 == 0) a.tri_count[sid] = 0;
-      } else if (a.tri_count[sid] > a.T) {
+      } else if (a.tri_count[sid] > max(a.T, a.T_ahead)) {
         // clipped again it would be the same cell, past T again
         if (l8 == 0) {
           a.status[sid] = kTriangleOverflow;

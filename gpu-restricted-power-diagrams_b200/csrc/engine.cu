@@ -545,7 +545,7 @@ int run_pass(rpd_solver *s, const int *ids, int num, int K, int P, int V, int T,
     if (a.hand.recs) cudaMemcpyAsync(hctr, a.hand.ctr, sizeof(hctr), cudaMemcpyDeviceToHost, st);
     if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return map_cuda(ctx, e, "cell kernel");
     const int parked = ctrs[0];
-    if (a.T_ahead > 0) s->ahead_max = ctrs[3];
+    if (a.T_ahead > 0) s->ahead_max = std::max(s->ahead_max, ctrs[3]);
     if (parked > a.defer.capacity || hctr[2] > 0) {
       CellLaunch b = a;
       b.hand = ClipHand();
@@ -1117,7 +1117,11 @@ static int launch_impl(rpd_solver *s, const rpd_params *pp, const PartSpec *part
       if (P > kMaxP || knn_slots(K) < 0) break;  // the reference stops at P >= 256 (voronoi.cpp:867)
       V = std::min(V, kMaxV);
       T = std::min(T, kMaxT);
-      if ((rc = run_pass(s, Cc, n1, K, P, V, T, eps, out_domain, counters, early)) != RPD_OK) return rc;
+      // triangle overflows settled ahead here too: the retries after this
+      // pass surely run while the cell fails
+      const int T_later = T_ahead > 0 ? t_ahead_cap(P, K, T, p.max_extra_passes - step - 1) : 0;
+      if ((rc = run_pass(s, Cc, n1, K, P, V, T, eps, out_domain, counters, early, 0, T_later, out_domain)) != RPD_OK)
+        return rc;
       if ((rc = recompute_ids(s, A, n0, 1, B, Cc, n0, n1, hist)) != RPD_OK) return rc;
       std::swap(A, B);
       n0_all = n0;
@@ -1449,19 +1453,6 @@ size_t solver_device_bytes(const rpd_solver *s) {
 }
 
 int clip_hand_capacity(int num) { return std::min(num, 65536 + num / 8); }
-
-int t_ahead_cap(int P, int K, int T, int max_extra) {
-  int T_ahead = 0;
-  for (int j = 0; j < max_extra; ++j) {
-    const int Pn = int(P * 1.5), Kn = int(K * 1.5);
-    if (Pn > kMaxP || knn_slots(Kn) < 0) break;
-    P = Pn;
-    K = Kn;
-    T = std::min(int(T * 1.5), kMaxT);
-    T_ahead = T;
-  }
-  return T_ahead;
-}
 
 }  // namespace rpd
 
