@@ -784,6 +784,8 @@ int capture(rpd_batch *b) {
   // (one untimed round first); the graph takes the faster.  Retry passes
   // (few rows) take a warp per seed.
   int variant[kKnnClasses];
+  // above K = 32 a warp per seed is always the faster (knn_variant_for)
+  auto trial_class = [&](int c) { return kKnnClassSlots[c] == 1 && class_rows[c] >= 16384; };
   for (int c = 0; c < kKnnClasses; ++c) {
     variant[c] = kKnnWarp;
     b->stats_trial_ms[c][0] = b->stats_trial_ms[c][1] = 0.f;
@@ -791,7 +793,7 @@ int capture(rpd_batch *b) {
   {
     bool trial = false;
     for (int c = 0; c < kKnnClasses; ++c)
-      trial |= class_used[c] && 32 * kKnnClassSlots[c] <= kKnnThreadMaxK && class_rows[c] >= 16384;
+      trial |= class_used[c] && trial_class(c);
     if (trial) {
       if (nprobe) {
         if ((e = probe_batch_launch(b->d_probes.as<ProbeLaunch>(), b->d_probe_start.as<int>(), nprobe, probe_rows,
@@ -819,7 +821,7 @@ int capture(rpd_batch *b) {
       for (auto &x : te) cudaEventCreate(&x);
       for (int c = 0; c < kKnnClasses; ++c) {
         const int S = kKnnClassSlots[c];
-        if (!class_used[c] || 32 * S > kKnnThreadMaxK || class_rows[c] < 16384) continue;
+        if (!class_used[c] || !trial_class(c)) continue;
         for (int round = 0; round < 2 && e == cudaSuccess; ++round) {
           if (round) cudaEventRecord(te[0], st);
           e = knn_batch_launch(S, pl.knn, pl.kstart + c * stride, nd, knn_blocks, st, -1, kKnnWarp);

@@ -389,12 +389,19 @@ int run_probe(rpd_solver *s, int P, int V, float eps, int *ids, int &nmiss, int 
 
 // The neighbour-search variant for K rows of this solver (rpd::KnnVariant).
 // RPD_FLAG_KNN_WARP / RPD_FLAG_KNN_THREAD force one.  Otherwise the
-// context's choice for K, made the first time K comes up with enough rows to
-// tell: both variants run on the first rows (one untimed round, one timed
-// with events), into `out`, which the real launch then overwrites; both give
-// the same lists, so only their speed differs.  Fewer rows than a trial
-// takes (retry passes): a warp per seed -- a thread per seed leaves most of
-// the GPU idle there and each row's search serial (0.45 ms for 144 rows).
+// context's choice for K.  Above kKnnTrialMaxK a warp per seed: it was the
+// faster of the two on every input measured (K 50: 1.90 against 3.04 ms for 1M
+// lattice seeds, 1.00 / 1.82 for 500K uniform ones, 0.23 / 0.58 for 100K).
+// Up to it, a trial the first time K comes up with enough rows to tell: both
+// variants run on the first quarter of the rows (a thread per seed needs
+// some 100K rows to fill the GPU: K 20, 0.18 / 0.21 ms for 100K seeds but 3.1
+// / 2.1 ms for 2M), one untimed round, one timed with events, into `out`,
+// which the real launch then overwrites; both give the same lists, so only
+// their speed differs.  Fewer rows than a trial takes (retry passes): a warp
+// per seed -- a thread per seed leaves most of the GPU idle there and each
+// row's search serial (0.45 ms for 144 rows).
+constexpr int kKnnTrialMaxK = 32;
+
 int knn_variant_for(rpd_solver *s, const int *ids, int num, int K, unsigned *out, unsigned flags) {
   if (flags & RPD_FLAG_KNN_WARP) return kKnnWarp;
   if (flags & RPD_FLAG_KNN_THREAD) return K <= kKnnThreadMaxK ? kKnnThread : kKnnWarp;
@@ -402,7 +409,8 @@ int knn_variant_for(rpd_solver *s, const int *ids, int num, int K, unsigned *out
   if (K > kKnnThreadMaxK || num < kTrialRows) return kKnnWarp;
   rpd_context *ctx = s->ctx;
   if (ctx->knn_variant[K] >= 0) return ctx->knn_variant[K];
-  const int m = kTrialRows;
+  if (K > kKnnTrialMaxK) return ctx->knn_variant[K] = kKnnWarp;
+  const int m = std::max(kTrialRows, std::min(num / 4, 262144));
   cudaStream_t st = ctx->stream;
   Events<4> ev;
   float ms[2] = {0.f, 0.f};
