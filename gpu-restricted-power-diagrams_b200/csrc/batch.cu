@@ -52,6 +52,8 @@ struct DiagStatic {
   double *hess;
   int *hessid;
   int H, HC;
+  AheadRecord *ahead;  // n: cells clipped past the first pass's caps (null: off)
+  int Kx0;         // neighbours per row of the first pass's table
   int *tri_count;  // n: the triangle overflows' counts (CellLaunch::tri_count; null: none)
   int safe_radius;  // the weighted security-radius guard (RPD_FLAG_SAFE_RADIUS)
   float cube_eps;
@@ -74,6 +76,7 @@ struct DiagState {
   const int *rc_ids;  // rows of the recompute (null: every cell)
   int rc_cond;        // 1: empty cells are not re-solved
   int hist[16];       // status histogram of the failing cells of the last recompute
+  int lP, lV;         // growths of P and V so far
   int ahead_max;      // the largest triangle count the first pass parked ahead
   int probe_outside;  // seeds the outside probe proved empty
   int final_hist[16]; // status histogram of every cell at the end
@@ -158,6 +161,7 @@ __global__ void __launch_bounds__(1024) k_plan(const DiagStatic *__restrict__ ds
       s.rc_cond = 0;
       s.rc_num = g.n;
       s.ahead_max = 0;
+      s.lP = s.lV = 0;
       continue;
     }
     if (!s.active) continue;
@@ -180,6 +184,8 @@ __global__ void __launch_bounds__(1024) k_plan(const DiagStatic *__restrict__ ds
           s.unfinished = 1;
           go = false;
         } else {
+          s.lP += s.hist[kPlaneOverflow] ? 1 : 0;
+          s.lV += s.hist[kVertexOverflow] ? 1 : 0;
           s.K = K;
           s.P = P;
           s.V = V;
@@ -225,7 +231,7 @@ __global__ void __launch_bounds__(1024) k_plan(const DiagStatic *__restrict__ ds
           koff += need;
         }
       }
-      const int c = s.active ? slot_class(s.K) : -1;
+      const int c = s.active ? slot_class(pa.pass == 0 ? g.Kx0 : s.K) : -1;
       for (int q = 0; q < kKnnClasses; ++q) {
         pl.kstart[q * stride + d] = kc[q];
         if (q == c) kc[q] += s.num;
@@ -266,7 +272,8 @@ __global__ void __launch_bounds__(1024) k_plan(const DiagStatic *__restrict__ ds
     kd.stored = g.stored;
     kd.counters = g.bins;
     kd.dim = g.dim;
-    kd.K = s.K;
+    kd.K = pa.pass == 0 ? g.Kx0 : s.K;
+    kd.skip = pa.pass == 0 ? nullptr : g.ahead;
     kd.ids = ids;
     kd.ring_bound = g.ring_bound;
     kd.out = kout;
@@ -275,6 +282,16 @@ __global__ void __launch_bounds__(1024) k_plan(const DiagStatic *__restrict__ ds
     a.n = g.n;
     a.knn = kout;
     a.K = s.K;
+    a.Kx = kd.K;
+    a.ahead = g.ahead;
+    a.ahead_first = pa.pass == 0 ? 1 : 0;
+    a.lP = s.lP;
+    a.lV = s.lV;
+    if (g.ahead && pa.pass == 0)
+      for (int k = 0, P = g.P0, V = g.V0; k < kAheadLevels; ++k, P = int(P * 1.5), V = min(int(V * 1.5), kMaxV)) {
+        a.ladP[k] = P;
+        a.ladV[k] = V;
+      }
     a.ids = ids;
     a.num = s.num;
     a.P = s.P;
@@ -396,6 +413,8 @@ __global__ void k_final_hist(const DiagStatic *__restrict__ ds, DiagState *__res
       const int d = owner_of_row(all_start, ndiag, i);
       const int stt = ds[d].status[i - all_start[d]];
       if (stt >= 0 && stt < 16) key = d * 16 + stt;
+      // a recorded cell that no pass settled: failed, no moments
+      if (ds[d].ahead && stt != kSuccess) ds[d].out[i - all_start[d]] = make_double4(0.0, 0.0, 0.0, 0.0);
     }
     const unsigned grp = __match_any_sync(kFull, key);
     if (key >= 0 && lane == __ffs(grp) - 1) atomicAdd(&st[key >> 4].final_hist[key & 15], __popc(grp));
@@ -491,6 +510,8 @@ int describe(rpd_batch *b, std::vector<DiagStatic> &out) {
   rpd_context *ctx = b->ctx;
   cudaError_t e;
   out.assign(b->ndiag, DiagStatic{});
+  bool any_safe = false;
+  for (const rpd_params &p : b->params) any_safe |= (p.flags & RPD_FLAG_SAFE_RADIUS) != 0;
   for (int d = 0; d < b->ndiag; ++d) {
     rpd_solver *s = b->solvers[d];
     const rpd_params &p = b->params[d];
@@ -509,8 +530,16 @@ int describe(rpd_batch *b, std::vector<DiagStatic> &out) {
     if ((e = s->ids_a.ensure(sizeof(int) * n)) != cudaSuccess) return map_cuda(ctx, e, "alloc ids");
     if ((e = s->ids_b.ensure(sizeof(int) * n)) != cudaSuccess) return map_cuda(ctx, e, "alloc ids");
     if ((e = s->ids_c.ensure(sizeof(int) * n)) != cudaSuccess) return map_cuda(ctx, e, "alloc ids");
-    if ((e = s->knn.ensure(sizeof(unsigned) * size_t(n) * p.K)) != cudaSuccess) return map_cuda(ctx, e, "alloc knn");
     DiagStatic &g = out[d];
+    // cells clipped past the first pass's caps, as rpd_solver_launch does
+    // (any size: the batch's cells share the launches)
+    const bool ahead = ahead_pays(p.K, p.V) && !any_safe && p.hessian_h == 0 && p.max_extra_passes > 0 &&
+                       !(p.flags & RPD_FLAG_FIRST_PASS_ONLY);
+    if (ahead && (e = s->ahead.ensure(sizeof(AheadRecord) * size_t(n))) != cudaSuccess)
+      return map_cuda(ctx, e, "alloc records");
+    g.ahead = ahead ? s->ahead.as<AheadRecord>() : nullptr;
+    g.Kx0 = ahead ? ahead_columns(p.K) : p.K;
+    if ((e = s->knn.ensure(sizeof(unsigned) * size_t(n) * g.Kx0)) != cudaSuccess) return map_cuda(ctx, e, "alloc knn");
     g.stored = s->stored.as<float4>();
     g.n = n;
     g.bins = s->counters.as<int>();
@@ -597,7 +626,7 @@ int capture(rpd_batch *b) {
   const std::vector<DiagStatic> &G = b->statics;
   long long cells = 0, table = 0;
   int Kmin = kMaxK, Kmax = 0, Pmax = 0, Vmax = 0, Tmax = 0, J = 0;
-  bool any_grid = false, any_plain = false, defer = true, any_safe = false, all_disjoint = true;
+  bool any_grid = false, any_plain = false, defer = true, any_safe = false, all_disjoint = true, any_ahead = false;
   int hess_hc = 0;  // the Hessian rows' HC of the diagrams that ask for rows (one for the batch)
   bool class_used[kKnnClasses] = {};
   long class_rows[kKnnClasses] = {};
@@ -607,7 +636,8 @@ int capture(rpd_batch *b) {
     const DiagStatic &g = G[d];
     all_start[d] = int(cells);
     cells += g.n;
-    table += (long long)g.n * g.K0;
+    table += (long long)g.n * g.Kx0;
+    any_ahead |= g.ahead != nullptr;
     Kmin = std::min(Kmin, g.K0);
     Kmax = std::max(Kmax, g.K0);
     Pmax = std::max(Pmax, g.P0);
@@ -627,7 +657,7 @@ int capture(rpd_batch *b) {
       defer = false;  // rows are summed in the cell's own warp
     }
     for (int c = 0; c < kKnnClasses; ++c)
-      if (knn_slots(g.K0) == kKnnClassSlots[c]) {
+      if (knn_slots(g.Kx0) == kKnnClassSlots[c]) {
         class_used[c] = true;
         class_rows[c] += g.n;
       }
@@ -932,6 +962,7 @@ int capture(rpd_batch *b) {
     cb.work = b->work.as<int>();
     cb.safe = any_safe;
     cb.hand = hand;
+    cb.ahead = j == 0 && any_ahead;
     if ((e = cell_batch_launch(cb, st, ctx->sm_count, &launches)) != cudaSuccess) return fail(e, "batch cells");
     // failing cells of the pass's diagrams
     k_fail_flags_batch<<<flat_blocks, 256, 0, st>>>(ds, sts, pl.rc_start, nd, b->f0.as<int>(), b->f1.as<int>());
@@ -1079,6 +1110,7 @@ int rpd_batch_launch(rpd_batch *b) {
     S.max_passes = std::max(S.max_passes, h.npasses);
     // with the probe the table holds the first pass's rows only
     s->knn_full_K = b->statics[d].probe ? 0 : b->params[d].K;
+    s->knn_full_Kx = b->statics[d].Kx0;
     s->used_on = false;
     s->used_count = -1;
     s->hess_h = b->statics[d].H;

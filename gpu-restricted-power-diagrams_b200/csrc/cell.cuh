@@ -83,11 +83,44 @@ struct ClipHand {
   int *ctr = nullptr;
 };
 
+// What a cell that failed a cap of the first pass needs, known since the
+// clipping went on past it (CellLaunch::ahead): the retry passes settle the
+// cell from this record instead of clipping it again.
+constexpr int kAheadLevels = 6;  // caps of the schedule: the first pass's, grown x1.5 one to five times
+struct AheadRecord {
+  unsigned short need;  // neighbours it takes to the security radius (0: no record)
+  // the neighbour at which the cap of each level stops the clipping (255: it
+  // does not): before its plane test, and at its cut
+  unsigned char jP[kAheadLevels], jV[kAheadLevels];
+  unsigned short pad;
+};
+static_assert(sizeof(AheadRecord) == 16, "ahead record size");
+
+// The status of a recorded cell in a pass of K neighbours and cap levels lP
+// and lV: the first cap that stops it decides.
+__host__ __device__ inline int ahead_status(const AheadRecord &r, int K, int lP, int lV) {
+  const int p = lP < kAheadLevels ? r.jP[lP] : 255, v = lV < kAheadLevels ? r.jV[lV] : 255;
+  const int first = p < v ? p : v, end = K < r.need ? K : r.need;
+  if (first < end) return p <= v ? kPlaneOverflow : kVertexOverflow;
+  return r.need <= K ? kSuccess : kSecurityRadiusNotReached;
+}
+
+// Whether a first pass of these caps clips past them, and the neighbours its
+// rows hold then.  Measured: with tight caps 30 to 95% of the cells fail it,
+// and the two passes that clip them again cost more than larger shared memory
+// and neighbour rows -- 2M blue-noise seeds (K 20, P 25, V 30, 94% failing)
+// 53.3 -> 37.4 ms on the device.  At K 50 .. 70, P 30, V 40 a few percent
+// fail, and clipping past the caps loses: 1M weighted seeds 11.7 -> 12.7 ms,
+// 100K 4.20 -> 4.42 ms.
+__host__ __device__ inline bool ahead_pays(int K, int V) { return K <= 24 || (V <= 32 && K <= 200); }
+__host__ __device__ inline int ahead_columns(int K) { return K <= 24 ? 48 : K; }
+
 struct CellLaunch {
   const float4 *stored = nullptr;  // n seeds in stored order (reference frame)
   int n = 0;
   const unsigned *knn = nullptr;   // num rows of K stored neighbour ids
   int K = 0;
+  int Kx = 0;                      // neighbours per row of knn (K, or more with ahead)
   const int *ids = nullptr;        // stored ids of the rows (null: row i = seed i)
   int num = 0;
   int P = 0, V = 0, T = 0;         // caps of this pass
@@ -142,6 +175,14 @@ struct CellLaunch {
   int *hessid = nullptr;
   int H = 0, HC = 1;
   ClipHand hand;  // recs == null: clip with a warp per cell
+  // Records of the cells clipped past the first pass's caps (n, stored order;
+  // null: off).  The first pass (ahead_first) writes every row's; the later
+  // ones settle the rows that have one.  Not with counters, used cells,
+  // Hessian rows or launches of one pass.
+  AheadRecord *ahead = nullptr;
+  int ahead_first = 0;
+  int lP = 0, lV = 0;              // levels of P and V
+  int ladP[kAheadLevels] = {}, ladV[kAheadLevels] = {};
 };
 constexpr int kParkOverflow = 101;  // internal status: the queue was full
 constexpr int kProbeMiss = 102;     // internal status: the outside probe proved nothing
@@ -242,6 +283,7 @@ struct CellBatch {
   int HC = 0;           // Hessian rows' components (a diagram with rows; then no defer queue), else 0
   bool disjoint = false;  // every diagram's grid lists each triangle in one voxel (a smaller id buffer)
   ClipHand hand;          // recs != null: clip with eight lanes per cell (the records' hand too)
+  bool ahead = false;     // a first pass with diagrams that clip past their caps (CellLaunch::ahead)
 };
 cudaError_t cell_batch_launch(const CellBatch &b, cudaStream_t st, int sm_count, int *launches = nullptr);
 // The same with the guard compiled in (cell_safe.cu).

@@ -2584,6 +2584,20 @@ __device__ __forceinline__ void finish_cell(WarpCell &w, const CellLaunch &a, co
   }
 }
 
+// Ahead records at the start of a row: the first pass clears the cell's, a
+// later one settles a cell that has one (true), whose moments are written
+// already.
+__device__ __forceinline__ bool settle_ahead(const CellLaunch &a, int sid, bool lead) {
+  if (a.ahead_first) {
+    if (lead) a.ahead[sid].need = 0;
+    return false;
+  }
+  const AheadRecord r = a.ahead[sid];
+  if (r.need == 0) return false;
+  if (lead) a.status[sid] = ahead_status(r, a.K, a.lP, a.lV);
+  return true;
+}
+
 // One row of a cell launch (one warp): clip, restrict, integrate, write.
 // `only_status` >= 0: skip the row unless its cell has that status; vc:
 // the vertex capacity (vertex_capacity).
@@ -2616,6 +2630,7 @@ __device__ __forceinline__ void cell_row(const CellLaunch &a, const Layout &L, u
       }
     }
   }
+  if (a.ahead && settle_ahead(a, sid, lane == 0)) return;
   const float4 s = a.stored[sid];
   double *tr = (a.trace && sid == a.trace_seed) ? a.trace : nullptr;
   const int trcap = a.trace_cap;
@@ -2647,7 +2662,7 @@ __device__ __forceinline__ void cell_row(const CellLaunch &a, const Layout &L, u
   if (track_nb && lane < 6) w.pnb[lane] = -1;
 
   // ---- power clipping by the K nearest, in order ----
-  const unsigned *nrow = a.knn + size_t(row) * a.K;
+  const unsigned *nrow = a.knn + size_t(row) * a.Kx;
   bool reached = false, exhausted = false, outside = false;
   const bool early = GRID && a.early_out && a.grid.sat != nullptr && a.wmin != nullptr && a.border_d == 0;
   double plain2 = early ? plain_radius2(a.grid, s, lane) : -1.0;

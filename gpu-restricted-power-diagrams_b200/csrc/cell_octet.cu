@@ -12,15 +12,20 @@ bool octet_applies(const CellLaunch &a) {
 
 namespace {
 
-template <int MW, bool GRID>
-cudaError_t launch_clip(const CellLaunch &a, cudaStream_t st) {
-  const OctLayout O = oct_layout<MW>(a.P, a.V);
+template <int MW, bool GRID, bool AHEAD>
+cudaError_t launch_clip_ahead(const CellLaunch &a, cudaStream_t st) {
+  const OctLayout O = oct_layout<MW>(a.P, a.V, AHEAD);
   const int threads = 128, cells = threads / kOct;
   const size_t smem = size_t(O.total) * cells;
-  cudaError_t e = allow_smem(reinterpret_cast<const void *>(k_clip<MW, GRID>), smem);
+  cudaError_t e = allow_smem(reinterpret_cast<const void *>(k_clip<MW, GRID, AHEAD>), smem);
   if (e != cudaSuccess) return e;
-  k_clip<MW, GRID><<<(a.num + cells - 1) / cells, threads, smem, st>>>(a, O);
+  k_clip<MW, GRID, AHEAD><<<(a.num + cells - 1) / cells, threads, smem, st>>>(a, O);
   return cudaGetLastError();
+}
+
+template <int MW, bool GRID>
+cudaError_t launch_clip(const CellLaunch &a, cudaStream_t st) {
+  return a.ahead && a.ahead_first ? launch_clip_ahead<MW, GRID, true>(a, st) : launch_clip_ahead<MW, GRID, false>(a, st);
 }
 
 template <int VS, bool GRID, bool INL>
@@ -56,13 +61,13 @@ cudaError_t launch_octet_vs(const CellLaunch &a, const Layout &L, cudaStream_t s
   return cudaGetLastError();
 }
 
-template <int MW, bool GRID>
-cudaError_t batch_clip(const CellBatch &b, const CellLaunch *descs, const int *start, long rows, cudaStream_t st,
-                       int sm_count) {
-  const OctLayout O = oct_layout<MW>(b.P, b.V);
+template <int MW, bool GRID, bool AHEAD>
+cudaError_t batch_clip_ahead(const CellBatch &b, const CellLaunch *descs, const int *start, long rows, cudaStream_t st,
+                             int sm_count) {
+  const OctLayout O = oct_layout<MW>(b.P, b.V, AHEAD);
   const int threads = 128, cells = threads / kOct;
   const size_t smem = size_t(O.total) * cells;
-  auto k = k_clip_batch<MW, GRID>;
+  auto k = k_clip_batch<MW, GRID, AHEAD>;
   cudaError_t e = allow_smem(reinterpret_cast<const void *>(k), smem);
   if (e != cudaSuccess) return e;
   int blocks;
@@ -76,6 +81,13 @@ cudaError_t batch_clip(const CellBatch &b, const CellLaunch *descs, const int *s
   }
   k<<<blocks, threads, smem, st>>>(descs, start, b.ndiag, O, work);
   return cudaGetLastError();
+}
+
+template <int MW, bool GRID>
+cudaError_t batch_clip(const CellBatch &b, const CellLaunch *descs, const int *start, long rows, cudaStream_t st,
+                       int sm_count) {
+  return b.ahead ? batch_clip_ahead<MW, GRID, true>(b, descs, start, rows, st, sm_count)
+                 : batch_clip_ahead<MW, GRID, false>(b, descs, start, rows, st, sm_count);
 }
 
 template <int VS, bool GRID, bool INL>

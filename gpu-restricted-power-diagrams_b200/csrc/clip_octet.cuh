@@ -30,6 +30,11 @@
 // evaluation adds 3u (|p|_1 + |d|); kTestErr takes 16u (sqrt(3) R + |d|), R
 // the cell's radius.
 //
+// AHEAD (CellLaunch::ahead, where ahead_pays): a first pass with tight caps
+// goes on past them and writes what the cell needs, so that the retry passes
+// need not clip it again: 2M blue-noise seeds' pass 1 10.3 -> 20.4 ms, passes
+// 2 to 5 29.2 -> 4.4 ms.
+//
 // Vertices keep the warp kernel's positions (holes filled by survivors in
 // order, then by the new vertices in boundary order), so that the cell's
 // later sums add the same terms in the same order.
@@ -70,13 +75,23 @@ struct OctCell {
   float4 s;
   Plane pl[kOct];
   float4 cand[kOct];
+  // clipping past the caps (CellLaunch::ahead): the status under the caps (-1:
+  // none of them reached), the last neighbour, and the record's levels
+  int vst, last;
+  unsigned char jP[kAheadLevels], jV[kAheadLevels], lP, lV;
+  unsigned char pad[2];
 };
 
+// ahead: room to clip past caps P and V.
 template <int MW>
-__host__ __device__ inline OctLayout oct_layout(int P, int V) {
+__host__ __device__ inline OctLayout oct_layout(int P, int V, bool ahead = false) {
   OctLayout L;
+  if (ahead) {
+    P = P < 32 * MW ? 32 * MW : P;
+    V += 8;
+  }
   L.Pc = P < kOctP ? P : kOctP;
-  L.Vc = V < kOctV ? (V + 7) & ~7 : kOctV;
+  L.Vc = V < kOctV ? (V + (ahead ? 15 : 7)) & (ahead ? ~15 : ~7) : kOctV;
   unsigned o = 32u * L.Pc;
   L.o_vert = o; o += 16u * L.Vc;
   L.o_cand = o; o += align16(unsigned(sizeof(OctCell)));
@@ -243,8 +258,8 @@ __device__ __forceinline__ unsigned long long drop_bits(unsigned long long m, in
 // Whether neighbour i of the row lies past twice the radius (the FP64
 // clipping's own test, radius_reached).
 __device__ __noinline__ bool oct_past(const CellLaunch &a, int row, int i, float4 s, double R2) {
-  if (i < 0 || i >= a.K) return false;
-  const unsigned z = __ldg(&a.knn[size_t(row) * a.K + i]);
+  if (i < 0 || i >= a.Kx) return false;
+  const unsigned z = __ldg(&a.knn[size_t(row) * a.Kx + i]);
   return z != kNone && seed_dist2(__ldg(&a.stored[z]), s) > 4.0 * R2;
 }
 
@@ -271,7 +286,9 @@ __device__ __noinline__ void oct_finish(const CellLaunch &a, const OctLayout &L,
   auto oct_bits = [&](bool p) { return (__ballot_sync(kFull, p) >> osh) & 0xffu; };
   const bool work = flags & kFinWork, reclip = flags & kFinReclip, odd = flags & kFinOdd, inside = flags & kFinInside;
   const int sid = work ? (a.ids ? a.ids[row] : row) : 0;
-  const float4 s = reinterpret_cast<const OctCell *>(osm + L.o_cand)->s;
+  const OctCell &oc = *reinterpret_cast<const OctCell *>(osm + L.o_cand);
+  const float4 s = oc.s;
+  const int vst = oc.vst;  // >= 0: the cell passed a cap, its status for now
   bool ok = work && !reclip && status == kSuccess;
   bool hand = false, zero = false;  // goes on in a warp; mass 0
   if constexpr (GRID) {
@@ -352,7 +369,7 @@ __device__ __noinline__ void oct_finish(const CellLaunch &a, const OctLayout &L,
 #pragma unroll
       for (int o = 4; o > 0; o >>= 1) ntri += __shfl_xor_sync(kFull, ntri, o);
       if (open && ntri > 0) {
-        if (g.tsat && ntri > a.T && (ntri > a.T_ahead || !a.defer.slots)) {
+        if (g.tsat && ntri > a.T && (ntri > a.T_ahead || !a.defer.slots) && vst < 0) {
           if (a.tri_count && l8 == 0) a.tri_count[sid] = ntri;
           status = kTriangleOverflow;
           ok = false;
@@ -380,6 +397,11 @@ __device__ __noinline__ void oct_finish(const CellLaunch &a, const OctLayout &L,
     }
   } else {
     if (ok && a.hess) hand = true;
+  }
+  if (vst >= 0 && hand) {
+    // past a cap and with boundary triangles: left to the retry passes
+    status = vst;
+    ok = hand = false;
   }
   const bool sum = ok && !hand && !zero;
   double acc[4] = {0, 0, 0, 0};
@@ -416,14 +438,25 @@ __device__ __noinline__ void oct_finish(const CellLaunch &a, const OctLayout &L,
       atomicAdd(&a.hand.ctr[2], 1);
       return;
     }
-    a.status[sid] = status;
-    a.out[sid] = status == kSuccess ? global_moments(acc, s) : make_double4(0.0, 0.0, 0.0, 0.0);
+    a.status[sid] = ok && vst >= 0 ? vst : status;
+    a.out[sid] = ok ? global_moments(acc, s) : make_double4(0.0, 0.0, 0.0, 0.0);
+    if (ok && vst >= 0) {
+      AheadRecord r;
+      r.need = (unsigned short)(oc.last + 1);
+      for (int k = 0; k < kAheadLevels; ++k) {
+        r.jP[k] = oc.jP[k];
+        r.jV[k] = oc.jV[k];
+      }
+      r.pad = 0;
+      a.ahead[sid] = r;
+    }
   }
 }
 
 // One cell per octet: clip, and where the cell needs no boundary triangles,
 // restrict, integrate and write.  act: the octet has row `row` of a.
-template <int MW, bool GRID>
+// AHEAD: launches with a first pass that clips past its caps (a.ahead).
+template <int MW, bool GRID, bool AHEAD>
 __device__ __forceinline__ void clip_octet(const CellLaunch &a, const OctLayout &L, unsigned char *osm, int row,
                                            bool act, int lane) {
   const int l8 = lane & 7;
@@ -444,8 +477,9 @@ __device__ __forceinline__ void clip_octet(const CellLaunch &a, const OctLayout 
   if (act) {
     const int sid = a.ids ? a.ids[row] : row;
     s = __ldg(&a.stored[sid]);
+    if (a.ahead && settle_ahead(a, sid, l8 == 0)) run = false;
     if (a.hess && l8 == 0) a.hessid[size_t(sid) * a.H] = -1;  // an empty row until the cell succeeds
-    if (GRID && a.tri_count) {
+    if (GRID && run && a.tri_count) {
       if (a.tri_first) {
         if (l8 == 0) a.tri_count[sid] = 0;
       } else if (a.tri_count[sid] > max(a.T, a.T_ahead)) {
@@ -468,9 +502,19 @@ __device__ __forceinline__ void clip_octet(const CellLaunch &a, const OctLayout 
   const bool work = run;  // the octet has a cell to clip
   // the neighbours' ids, a chunk ahead of their use
   unsigned zn = kNone;
-  auto fetch = [&](int i) { zn = run && i < a.K ? __ldg(&a.knn[size_t(row) * a.K + i]) : kNone; };
+  const bool ahead = AHEAD && work && a.ahead && a.ahead_first;
+  const int Kend = ahead ? a.Kx : a.K;  // neighbours at hand
+  auto fetch = [&](int i) { zn = run && i < Kend ? __ldg(&a.knn[size_t(row) * a.Kx + i]) : kNone; };
   fetch(l8);
-  if (l8 == 0) oc.s = s;
+  if (l8 == 0) {
+    oc.s = s;
+    oc.vst = -1;
+    if (ahead) {
+      for (int k = 0; k < kAheadLevels; ++k) oc.jP[k] = oc.jV[k] = 255;
+      oc.lP = oc.lV = 0;
+    }
+  }
+  int vst = -1;  // the status under the caps, once one of them is passed
   // the domain box
   if (l8 < 6) plane[l8] = box_plane(s, work ? a.cube_eps : 0.f, l8);
   __syncwarp();
@@ -484,7 +528,8 @@ __device__ __forceinline__ void clip_octet(const CellLaunch &a, const OctLayout 
   }
   __syncwarp();
   int np = 6, nv = 8;
-  const int Pm = work ? min(a.P, kOctP) : 0;
+  const int Pm = !work ? 0 : (ahead ? L.Pc : min(a.P, kOctP));
+  const int Vm = ahead ? L.Vc : min(a.V, kOctV);
   bool reclip = false;    // the caps here do not hold the cell: the warp kernel clips it
   bool inside = false;    // the seed surely lies in its own cell (nonempty_cell)
   bool cut = false;
@@ -529,7 +574,6 @@ __device__ __forceinline__ void clip_octet(const CellLaunch &a, const OctLayout 
   // the chunk's first neighbour that needs more than a test: past the chunk,
   // past the row, or with the planes used up (0 before the first chunk)
   int lim = 0;
-  const int K = work ? a.K : 0;
   int smax = kOct;  // at least every octet's vertex count
   for (;;) {
     // ---- the next neighbour that cuts, for every octet ----
@@ -558,15 +602,29 @@ __device__ __forceinline__ void clip_octet(const CellLaunch &a, const OctLayout 
         __syncwarp();
         vbits = oct_bits(valid);
         stops();
-        lim = np >= Pm ? 0 : (vbits == 0xffu ? kOct : __ffs(~vbits) - 1);
+        auto limit = [&]() {
+          lim = np >= Pm || (AHEAD && ahead && vst < 0 && np >= a.P) ? 0 : (vbits == 0xffu ? kOct : __ffs(~vbits) - 1);
+          if (AHEAD && ahead && vst < 0) lim = min(lim, max(a.K - i0, 0));
+        };
+        limit();
         if (need && jj >= lim) {
-          if (i0 + jj >= K) {
-            status = kSecurityRadiusNotReached;
-          } else if ((vbits >> jj) & 1u) {
-            if (np >= a.P) status = kPlaneOverflow;
+          const int i = i0 + jj;
+          const bool there = i < Kend && ((vbits >> jj) & 1u);
+          if (AHEAD && ahead && vst < 0) {
+            if (i >= a.K) vst = kSecurityRadiusNotReached;
+            else if (there && np >= a.P) vst = kPlaneOverflow;
+          }
+          bool on = false;
+          if (i >= Kend) {
+            status = AHEAD && vst >= 0 ? vst : kSecurityRadiusNotReached;
+          } else if (there) {
+            if (np < Pm) on = AHEAD;  // past a cap only
+            else if (AHEAD && vst >= 0) status = vst;
+            else if (np >= a.P) status = kPlaneOverflow;
             else reclip = true;
           }  // else fewer than K other seeds: all have been clipped
-          run = need = false;
+          if (AHEAD && on) limit();
+          else run = need = false;
         }
       }
       const float4 e = oc.cand[jj & 7];
@@ -607,7 +665,7 @@ __device__ __forceinline__ void clip_octet(const CellLaunch &a, const OctLayout 
       if (need) rm = rt;
       cut |= need && rt != 0;
       run = run && !(need && rt == 0 && past);  // reached
-      jj += need && rt == 0 ? 1 : 0;
+      jj += need && rt == 0 && !past ? 1 : 0;
     }
     if (!__any_sync(kFull, cut)) break;
     // ---- the cut ----
@@ -622,7 +680,7 @@ __device__ __forceinline__ void clip_octet(const CellLaunch &a, const OctLayout 
     // kernel's order (clip): its directed edges whose twin is not in it
     const bool from_kept = min(nrem, nkeep) <= 10 && nkeep < nrem;
     if (cut && nkeep == 0) {
-      status = kEmptyCell;
+      status = AHEAD && vst >= 0 ? vst : kEmptyCell;
       run = cut = false;
     }
     const unsigned long long side = cut ? (from_kept ? ~rm & live : rm) : 0ull;
@@ -736,11 +794,20 @@ __device__ __forceinline__ void clip_octet(const CellLaunch &a, const OctLayout 
     bad = oct_bits(bad) != 0;
     const int F = nkeep + nb;
     if (cut && bad) {
-      status = kInconsistentBoundary;
+      status = AHEAD && vst >= 0 ? vst : kInconsistentBoundary;
       run = cut = false;
     }
-    if (cut && F > min(a.V, kOctV)) {
-      if (F > a.V) status = kVertexOverflow;
+    if (AHEAD && ahead && cut) {
+      // the levels that this cut passes
+      if (F > a.V && vst < 0) vst = kVertexOverflow;
+      if (l8 == 0) {
+        while (oc.lV < kAheadLevels && F > a.ladV[oc.lV]) oc.jV[oc.lV++] = (unsigned char)(i0 + jj);
+        while (oc.lP < kAheadLevels && pid + 1 >= a.ladP[oc.lP]) oc.jP[oc.lP++] = (unsigned char)(i0 + jj + 1);
+      }
+    }
+    if (cut && F > Vm) {
+      if (AHEAD && vst >= 0) status = vst;
+      else if (F > a.V) status = kVertexOverflow;
       else reclip = true;
       run = cut = false;
     }
@@ -781,7 +848,7 @@ __device__ __forceinline__ void clip_octet(const CellLaunch &a, const OctLayout 
     if (rare(__any_sync(kFull, degenerate || od))) {
       odd |= oct_bits(od) != 0;
       if (oct_bits(degenerate) != 0 && cut) {
-        status = kInconsistentBoundary;
+        status = AHEAD && vst >= 0 ? vst : kInconsistentBoundary;
         run = cut = false;
       }
     }
@@ -789,7 +856,7 @@ __device__ __forceinline__ void clip_octet(const CellLaunch &a, const OctLayout 
       nv = F;
       np = pid + 1;
     }
-    if (np >= Pm) lim = 0;
+    if (np >= Pm || (AHEAD && ahead && np >= a.P)) lim = 0;
     smax = __reduce_max_sync(kFull, run ? nv : 0);
     radius(smax);
     stops();
@@ -802,23 +869,28 @@ __device__ __forceinline__ void clip_octet(const CellLaunch &a, const OctLayout 
 
   const unsigned flags = (work ? kFinWork : 0u) | (reclip ? kFinReclip : 0u) | (odd ? kFinOdd : 0u) |
                          (inside ? kFinInside : 0u);
+  if (AHEAD && ahead && l8 == 0) {
+    oc.vst = vst;
+    oc.last = i0 + jj;
+  }
+  __syncwarp();
   oct_finish<GRID>(a, L, osm, row, flags, status, np, nv, m2, lane);
 }
 
-template <int MW, bool GRID>
-__global__ void __launch_bounds__(128, MW == 1 ? 6 : 5)
+template <int MW, bool GRID, bool AHEAD>
+__global__ void __launch_bounds__(128, MW == 1 && !AHEAD ? 6 : 5)
     k_clip(const __grid_constant__ CellLaunch a, const __grid_constant__ OctLayout L) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int lane = threadIdx.x & 31;
   const int row = (blockIdx.x * blockDim.x + threadIdx.x) / kOct;
   if ((row & ~3) >= a.num) return;  // the whole warp
-  clip_octet<MW, GRID>(a, L, smem + size_t(threadIdx.x / kOct) * L.total, row, row < a.num, lane);
+  clip_octet<MW, GRID, AHEAD>(a, L, smem + size_t(threadIdx.x / kOct) * L.total, row, row < a.num, lane);
 }
 
 // The rows of many diagrams (k_cell_batch's scheme): diagram d owns rows
 // start[d] .. start[d+1].  work (optional, zeroed before the launch): warps
 // take four rows at a time from it; null: one octet per row.
-template <int MW, bool GRID>
+template <int MW, bool GRID, bool AHEAD>
 __global__ void __launch_bounds__(128, 5)
     k_clip_batch(const CellLaunch *__restrict__ descs, const int *__restrict__ start, int ndiag,
                  const __grid_constant__ OctLayout L, int *__restrict__ work) {
@@ -836,7 +908,7 @@ __global__ void __launch_bounds__(128, 5)
     const int r = r0 + lane / kOct;
     const bool act = r < total;
     const int d = owner_of_row(start, ndiag, act ? r : r0);
-    clip_octet<MW, GRID>(descs[d], L, osm, r - start[d], act, lane);
+    clip_octet<MW, GRID, AHEAD>(descs[d], L, osm, r - start[d], act, lane);
     if (!work) break;
     __syncwarp();
   }
@@ -861,7 +933,7 @@ __device__ __forceinline__ void finish_records(const ClipHand &hd, const Layout 
     const int row = r->row, np = r->np, nv = r->nv;
     const int sid = a.ids ? a.ids[row] : row;
     const float4 s = a.stored[sid];
-    const unsigned *nrow = a.knn + size_t(row) * a.K;
+    const unsigned *nrow = a.knn + size_t(row) * a.Kx;
     const bool track = (GRID && a.used) || (INL && a.hess);
     for (int i = lane; i < np; i += 32) {
       int z = -1;

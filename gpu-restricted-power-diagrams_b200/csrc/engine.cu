@@ -102,6 +102,36 @@ __global__ void k_fail_flags(const int *__restrict__ ids, int num, const int *__
   if (fail) atomicAdd(&hist[st], 1);
 }
 
+// Settles the listed cells that have a record (CellLaunch::ahead) in a pass of
+// K neighbours and cap levels lP and lV; the others go to `out`, *count of
+// them (zeroed before), every warp's in order.  Bound by memory latency; it
+// takes the settled rows out of the passes' kernels, which ran mostly empty
+// octets: 2M blue-noise seeds' passes 2 and 3 with the neighbour search
+// 12.8 -> 8.5 ms.
+__global__ void k_settle_ahead(const int *__restrict__ ids, int num, const AheadRecord *__restrict__ rec, int K, int lP,
+                               int lV, int *__restrict__ status, int *__restrict__ out, int *__restrict__ count) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
+  bool left = false;
+  int sid = 0;
+  if (i < num) {
+    sid = ids[i];
+    const AheadRecord r = rec[sid];
+    left = r.need == 0;
+    if (!left) status[sid] = ahead_status(r, K, lP, lV);
+  }
+  const unsigned m = __ballot_sync(kFull, left);
+  int base = 0;
+  if (lane == 0 && m) base = atomicAdd(count, __popc(m));
+  base = __shfl_sync(kFull, base, 0);
+  if (left) out[base + __popc(m & ((1u << lane) - 1u))] = sid;
+}
+
+__global__ void k_clear_failed(const int *__restrict__ ids, int num, const int *__restrict__ status,
+                               double4 *__restrict__ out) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < num && status[ids[i]] != kSuccess) out[ids[i]] = make_double4(0.0, 0.0, 0.0, 0.0);
+}
+
 __global__ void k_fail_scatter(const int *__restrict__ ids, int num, const int *__restrict__ f0,
                                const int *__restrict__ s0, const int *__restrict__ f1, const int *__restrict__ s1,
                                int *__restrict__ out0, int *__restrict__ out1, int *__restrict__ counts) {
@@ -450,19 +480,24 @@ int run_pass(rpd_solver *s, const int *ids, int num, int K, int P, int V, int T,
   // all cells with this K is kept across weight-only re-solves
   const bool all_cells = ids == nullptr && num == s->n;
   rpd::DevBuf &kb = all_cells ? s->knn : s->knn_part;
-  const bool reuse = all_cells && s->knn_full_K == K && !counters && !s->fresh_knn;
-  if ((e = kb.ensure(sizeof(unsigned) * size_t(num) * K)) != cudaSuccess) return map_cuda(ctx, e, "alloc knn");
+  const bool ahead_first = s->ahead_on && pi == 0;
+  const int Kx = ahead_first ? ahead_columns(K) : K;
+  const bool reuse = all_cells && s->knn_full_K == K && s->knn_full_Kx == Kx && !counters && !s->fresh_knn;
+  if ((e = kb.ensure(sizeof(unsigned) * size_t(num) * Kx)) != cudaSuccess) return map_cuda(ctx, e, "alloc knn");
   Events<4> ev;
   unsigned long long *ctr = counters ? s->counter64.as<unsigned long long>() : nullptr;
   cudaEventRecord(ev[0], st);
   if (!reuse) {
     if (all_cells) s->knn_full_K = 0;
-    const int variant = knn_variant_for(s, ids, num, K, kb.as<unsigned>(), s->launch_flags);
+    const int variant = knn_variant_for(s, ids, num, Kx, kb.as<unsigned>(), s->launch_flags);
     if (pi < 8) S.pass_knn_variant[pi] = variant;
-    e = knn_launch(s->stored.as<float4>(), s->counters.as<int>(), s->dim, ids, num, K, s->ring_bound.as<float>(),
+    e = knn_launch(s->stored.as<float4>(), s->counters.as<int>(), s->dim, ids, num, Kx, s->ring_bound.as<float>(),
                    kb.as<unsigned>(), ctr ? ctr + RPD_CTR_NUM : nullptr, st, variant);
     if (e != cudaSuccess) return map_cuda(ctx, e, "knn");
-    if (all_cells) s->knn_full_K = K;
+    if (all_cells) {
+      s->knn_full_K = K;
+      s->knn_full_Kx = Kx;
+    }
     S.kernel_launches += 1;
   }
   cudaEventRecord(ev[1], st);
@@ -471,6 +506,7 @@ int run_pass(rpd_solver *s, const int *ids, int num, int K, int P, int V, int T,
   a.n = s->n;
   a.knn = kb.as<unsigned>();
   a.K = K;
+  a.Kx = Kx;
   a.ids = ids;
   a.num = num;
   a.P = P;
@@ -532,6 +568,14 @@ int run_pass(rpd_solver *s, const int *ids, int num, int K, int P, int V, int T,
     dq.part = s->defer_part.as<double>();
     dq.fail = s->defer_fail.as<int>();
     dq.counters = s->defer_ctr.as<int>();
+  }
+  if (ahead_first) {  // later passes get rows without a record
+    a.ahead = s->ahead.as<AheadRecord>();
+    a.ahead_first = 1;
+    for (int k = 0; k < kAheadLevels; ++k) {
+      a.ladP[k] = s->lad_P[k];
+      a.ladV[k] = s->lad_V[k];
+    }
   }
   if (num >= kOctetMinRows && octet_applies(a)) {
     ClipHand &hd = a.hand;
@@ -822,6 +866,7 @@ int rpd_solver_knn(rpd_solver *s, int K, int *knn_user, rpd_mem where, float *de
   cudaEventRecord(ev[1], st);
   if (e != cudaSuccess) return map_cuda(ctx, e, "knn");
   s->knn_full_K = K;
+  s->knn_full_Kx = K;
   int *dst = where == RPD_DEVICE ? knn_user : s->knn_user.as<int>();
   const int tb = 256;
   k_knn_to_user<<<int((nk + tb - 1) / tb), tb, 0, st>>>(s->knn.as<unsigned>(), s->perm.as<int>(),
@@ -1094,6 +1139,19 @@ static int launch_impl(rpd_solver *s, const rpd_params *pp, const PartSpec *part
     if (count > 0) k_iota<<<(count + 255) / 256, 256, 0, st>>>(first, count, s->ids_range.as<int>());
     range = s->ids_range.as<int>();
   }
+  // cells clipped past the first pass's caps, so that the retries can settle
+  // them from a record (tight caps fail most cells)
+  s->ahead_on = ahead_pays(p.K, p.V) && !counters && !s->used_on && s->hess_h == 0 && !(p.flags & RPD_FLAG_SAFE_RADIUS) &&
+                s->precision <= 1 && p.max_extra_passes > 0 && !(p.flags & RPD_FLAG_FIRST_PASS_ONLY) &&
+                count >= kOctetMinRows;
+  if (s->ahead_on) {
+    if ((e = s->ahead.ensure(sizeof(AheadRecord) * size_t(n))) != cudaSuccess) return map_cuda(ctx, e, "alloc records");
+    s->level_P = s->level_V = 0;
+    for (int k = 0, P = p.P, V = p.V; k < kAheadLevels; ++k, P = int(P * 1.5), V = std::min(int(V * 1.5), kMaxV)) {
+      s->lad_P[k] = P;
+      s->lad_V[k] = V;
+    }
+  }
   if (probe) {
     int nmiss = 0;
     int *miss = s->ids_b.as<int>();
@@ -1115,8 +1173,8 @@ static int launch_impl(rpd_solver *s, const rpd_params *pp, const PartSpec *part
     if ((rc = reduce_schedule(s, part, hist, n0_all)) != RPD_OK) return rc;
     for (int step = 0; step < p.max_extra_passes && n0_all > 0; ++step) {
       bool relaunch = false;
-      if (hist[kVertexOverflow]) { relaunch = true; V = int(V * 1.5); }
-      if (hist[kPlaneOverflow]) { relaunch = true; P = int(P * 1.5); }
+      if (hist[kVertexOverflow]) { relaunch = true; V = int(V * 1.5); s->level_V++; }
+      if (hist[kPlaneOverflow]) { relaunch = true; P = int(P * 1.5); s->level_P++; }
       if (hist[kSecurityRadiusNotReached]) { relaunch = true; K = int(K * 1.5); }
       // cells parked ahead still fail in the reference's passes while T is
       // below their count, and keep T growing
@@ -1128,12 +1186,34 @@ static int launch_impl(rpd_solver *s, const rpd_params *pp, const PartSpec *part
       // triangle overflows settled ahead here too: the retries after this
       // pass surely run while the cell fails
       const int T_later = T_ahead > 0 ? t_ahead_cap(P, K, T, p.max_extra_passes - step - 1) : 0;
-      if ((rc = run_pass(s, Cc, n1, K, P, V, T, eps, out_domain, counters, early, 0, T_later, out_domain)) != RPD_OK)
+      const int *rows = Cc;
+      int nrows = n1;
+      if (s->ahead_on && n1 > 0) {
+        // recorded cells are settled here, the others (fail_ws holds their
+        // ids until the next recompute_ids) solved again
+        int *left = s->fail_ws.as<int>(), *count = s->hist.as<int>() + 15;
+        cudaMemsetAsync(count, 0, sizeof(int), st);
+        k_settle_ahead<<<(n1 + 255) / 256, 256, 0, st>>>(Cc, n1, s->ahead.as<AheadRecord>(), K, s->level_P, s->level_V,
+                                                        s->status.as<int>(), left, count);
+        s->stats.kernel_launches += 1;
+        if ((e = cudaMemcpyAsync(&nrows, count, sizeof(int), cudaMemcpyDeviceToHost, st)) != cudaSuccess ||
+            (e = cudaStreamSynchronize(st)) != cudaSuccess)
+          return map_cuda(ctx, e, "settle ahead");
+        rows = left;
+      }
+      const int pi = s->stats.npasses;
+      if ((rc = run_pass(s, rows, nrows, K, P, V, T, eps, out_domain, counters, early, 0, T_later, out_domain)) != RPD_OK)
         return rc;
+      if (pi < 8) s->stats.pass_cells[pi] = n1;  // the reference solves all of them again
       if ((rc = recompute_ids(s, A, n0, 1, B, Cc, n0, n1, hist)) != RPD_OK) return rc;
       std::swap(A, B);
       n0_all = n0;
       if ((rc = reduce_schedule(s, part, hist, n0_all)) != RPD_OK) return rc;
+    }
+    if (s->ahead_on && n0 > 0) {
+      // the recorded cells that no pass settled: failed, no moments
+      k_clear_failed<<<(n0 + 255) / 256, 256, 0, st>>>(A, n0, s->status.as<int>(), s->out.as<double4>());
+      s->stats.kernel_launches += 1;
     }
   }
   if (s->used_on) {
@@ -1294,7 +1374,7 @@ int rpd_solver_trace_cell(rpd_solver *s, int user_id, const rpd_params *pp, doub
   a.stored = s->stored.as<float4>();
   a.n = n;
   a.knn = s->knn_part.as<unsigned>();
-  a.K = p.K;
+  a.K = a.Kx = p.K;
   a.ids = id.as<int>();
   a.num = 1;
   a.P = p.P;
@@ -1444,6 +1524,7 @@ void solver_trim(rpd_solver *s) {
   s->defer_chunk_slot.release();
   s->hand_recs.release();
   s->hand_ctr.release();
+  s->ahead.release();
   s->hess.release();  // --hessian rows are read out before a trim
   s->hessid.release();
   s->hess_h = 0;
@@ -1454,7 +1535,7 @@ size_t solver_device_bytes(const rpd_solver *s) {
                        &s->ring_bound, &s->knn, &s->knn_part, &s->tri_count, &s->knn_user, &s->counter64, &s->g_flags, &s->g_points,
                        &s->g_tris, &s->g_list, &s->g_offsets, &s->g_sat, &s->g_tsat, &s->out, &s->status, &s->ids_a, &s->ids_b,
                        &s->ids_c, &s->fail_ws, &s->hist, &s->gather, &s->defer_slots, &s->defer_part, &s->defer_fail,
-                       &s->defer_ctr, &s->defer_chunk_slot, &s->hand_recs, &s->hand_ctr, &s->wmin, &s->used, &s->hess, &s->hessid};
+                       &s->defer_ctr, &s->defer_chunk_slot, &s->hand_recs, &s->hand_ctr, &s->ahead, &s->wmin, &s->used, &s->hess, &s->hessid};
   size_t t = 0;
   for (const DevBuf *x : b) t += x->bytes;
   return t;

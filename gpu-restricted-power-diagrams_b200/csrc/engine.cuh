@@ -82,6 +82,7 @@ struct rpd_solver {
   rpd::DevBuf ring_bound;      // float[dim+2]
   rpd::DevBuf knn;             // unsigned[n*K]: every cell's neighbours (stored ids)
   int knn_full_K = 0;          // K of the table in knn for all n cells (0: none)
+  int knn_full_Kx = 0;         // neighbours per row of that table
   int launches_since_points = 0;  // launches since the seeds were set (the outside probe runs on the first)
   long long grid_nonplain = -1;   // voxels of the grid that are not plainly outside (-1: not read yet)
   rpd::DevBuf knn_part;        // unsigned[num*K]: rows of a retry pass or a trace
@@ -102,6 +103,10 @@ struct rpd_solver {
   rpd::DevBuf gather;          // user-order staging for outputs
   rpd::DevBuf defer_slots, defer_part, defer_fail, defer_ctr, defer_chunk_slot;  // parked boundary cells
   rpd::DevBuf hand_recs, hand_ctr;  // cells handed from the octet clipping to a warp
+  rpd::DevBuf ahead;           // AheadRecord[n]: cells clipped past the first pass's caps
+  bool ahead_on = false;       // in the current launch
+  int level_P = 0, level_V = 0;                                  // growths of P and V so far
+  int lad_P[rpd::kAheadLevels] = {}, lad_V[rpd::kAheadLevels] = {};  // the caps after each
   int ahead_max = 0;           // the largest triangle count the first pass parked ahead
   bool have_results = false;
   bool use_defer = true;       // park heavy boundary cells for the chunked kernel

@@ -549,7 +549,9 @@ __global__ void __launch_bounds__(kThreadRows) k_knn_thread_batch(const KnnDiag 
     const int d = owner_of_row(start, ndiag, r);
     const KnnDiag &g = diags[d];
     const int i = r - start[d];
-    knn_thread_row(g.stored, g.counters, g.dim, g.ids ? g.ids[i] : i, g.K, g.ring_bound, H);
+    const int pin = g.ids ? g.ids[i] : i;
+    if (g.skip && g.skip[pin].need) continue;
+    knn_thread_row(g.stored, g.counters, g.dim, pin, g.K, g.ring_bound, H);
     unsigned *o = g.out + size_t(i) * g.K;
     for (int k = 0; k < g.K; ++k) o[k] = unsigned(H.at(k) & 0xffffffffull);
   }
@@ -569,6 +571,7 @@ __global__ void __launch_bounds__(256) k_knn_batch(const KnnDiag *__restrict__ d
     const KnnDiag &g = diags[d];
     const int i = r - start[d];
     const int pin = g.ids ? g.ids[i] : i;
+    if (g.skip && g.skip[pin].need) continue;
     knn_row<S>(g.stored, g.counters, g.dim, pin, g.K, g.ring_bound, g.out + size_t(i) * g.K, nullptr,
                buf[threadIdx.x >> 5], lane);
   }

@@ -1,6 +1,7 @@
 // K-nearest-neighbour search over binned seeds (one warp per seed).
 #pragma once
 #include "bins.cuh"
+#include "cell.cuh"
 
 namespace rpd {
 
@@ -37,6 +38,9 @@ struct KnnDiag {
   const int *ids;
   const float *ring_bound;
   unsigned *out;
+  // optional, by stored id: rows of seeds that have a record
+  // (AheadRecord::need) are left out, their entries unspecified
+  const AheadRecord *skip;
 };
 // Slot classes of knn_slots, in order.
 constexpr int kKnnClasses = 6;

@@ -107,14 +107,15 @@ size_t device_grid_build_bytes(int size) {
 // inverse, neighbour table, results, status, bins.
 size_t resident_bytes(int n, const rpd_params &p) {
   const size_t bins = size_t(double(n) / 3.1 * 1.2) + 64;
-  return size_t(n) * (16 + 16 + 4 + 4 + 32 + 4 + 4 * size_t(p.K)) + bins * 4 + 4096;
+  return size_t(n) * (16 + 16 + 4 + 4 + 32 + 4 + 4 * size_t(rpd::ahead_pays(p.K, p.V) ? rpd::ahead_columns(p.K) : p.K)) + bins * 4 + 4096;
 }
 
 // Device bytes a launch needs on top: binning workspace, failing-id lists,
 // staging, parked boundary cells, neighbour rows of retry passes (caps grown
 // x1.5 up to 5 times: bounded by 8x the first caps, which also bounds the
 // first pass's slots for triangle overflows parked ahead).  Per work item of
-// the parked cells: partial moments, failure, owning slot (40 bytes).
+// the parked cells: partial moments, failure, owning slot (40 bytes).  Records
+// of the cells handed to a warp, and of those clipped past the caps (16 bytes).
 size_t transient_bytes(int n, const rpd_params &p) {
   const size_t cap = std::min<size_t>(size_t(n), std::max<size_t>(32768, size_t(n) / 8));
   const size_t P = size_t(std::min(255, p.P * 8)), V = size_t(std::min(256, p.V * 8)),
@@ -122,7 +123,8 @@ size_t transient_bytes(int n, const rpd_params &p) {
   const size_t slot = 144 + 32 * P + 44 * V + 4 * T;
   // --hessian: the rows on the device and their user-order staging
   const size_t hess = p.hessian_h > 0 ? 2 * size_t(n) * size_t(p.hessian_h) * (8 * size_t(p.hessian_hc) + 4) : 0;
-  return size_t(n) * (12 + 16 + 32 + 12) + cap * (slot / 4 + 40 * (T / 32 + 1) / 4) +
+  return size_t(n) * (12 + 16 + 32 + 12 + 16) + cap * (slot / 4 + 40 * (T / rpd::kConeChunk + 1) / 4) +
+         size_t(rpd::clip_hand_capacity(n)) * rpd::kClipRecordBytes +
          size_t(n) / 4 * size_t(p.K) * 8 * 4 + hess + (size_t(1) << 20);
 }
 
