@@ -86,23 +86,25 @@ struct ClipHand {
 // What a cell that failed a cap of the first pass needs, known since the
 // clipping went on past it (CellLaunch::ahead): the retry passes settle the
 // cell from this record instead of clipping it again.
+constexpr int kMaxT = 4096;
 constexpr int kAheadLevels = 6;  // caps of the schedule: the first pass's, grown x1.5 one to five times
 struct AheadRecord {
   unsigned short need;  // neighbours it takes to the security radius (0: no record)
   // the neighbour at which the cap of each level stops the clipping (255: it
   // does not): before its plane test, and at its cut
   unsigned char jP[kAheadLevels], jV[kAheadLevels];
-  unsigned short pad;
+  unsigned short ntri;  // triangles its restriction needs, when more than the T of the recording pass (else 0)
 };
 static_assert(sizeof(AheadRecord) == 16, "ahead record size");
 
-// The status of a recorded cell in a pass of K neighbours and cap levels lP
-// and lV: the first cap that stops it decides.
-__host__ __device__ inline int ahead_status(const AheadRecord &r, int K, int lP, int lV) {
+// The status of a recorded cell in a pass of K neighbours, T triangles and
+// cap levels lP and lV: the first cap that stops it decides.
+__host__ __device__ inline int ahead_status(const AheadRecord &r, int K, int T, int lP, int lV) {
   const int p = lP < kAheadLevels ? r.jP[lP] : 255, v = lV < kAheadLevels ? r.jV[lV] : 255;
   const int first = p < v ? p : v, end = K < r.need ? K : r.need;
   if (first < end) return p <= v ? kPlaneOverflow : kVertexOverflow;
-  return r.need <= K ? kSuccess : kSecurityRadiusNotReached;
+  if (r.need > K) return kSecurityRadiusNotReached;
+  return r.ntri > T ? kTriangleOverflow : kSuccess;
 }
 
 // Whether a first pass of these caps clips past them, and the neighbours its
@@ -183,6 +185,13 @@ struct CellLaunch {
   int ahead_first = 0;
   int lP = 0, lV = 0;              // levels of P and V
   int ladP[kAheadLevels] = {}, ladV[kAheadLevels] = {};
+  // A retry pass of few cells (retry) takes Kx neighbours where a cell does
+  // not reach its radius with K, and parks cells of up to T_ahead triangles;
+  // a cell that needs more than K, or more than T_sure, gets a record and its
+  // status (kSuccess when all went well) is that of a later pass
+  // (k_retry_status puts this one's).
+  int retry = 0;
+  int T_sure = kMaxT;
 };
 constexpr int kParkOverflow = 101;  // internal status: the queue was full
 constexpr int kProbeMiss = 102;     // internal status: the outside probe proved nothing
@@ -193,7 +202,6 @@ constexpr int kTraceRecord = 12;
 // voronoi.cpp:867), V <= 256, T <= kMaxT.
 constexpr int kMaxP = 255;
 constexpr int kMaxV = 256;
-constexpr int kMaxT = 4096;
 
 // The T of the last retry pass that surely runs after a cell's triangle
 // overflow in a pass of these caps: passes grow T x1.5 while the cell fails,

@@ -2122,12 +2122,24 @@ __device__ void park_fixed(const DeferQueue &dq, int slot, int diag, int sid, in
   }
 }
 
+// The record of a cell of a retry pass (CellLaunch::retry), whose caps no
+// later pass's cells outgrow.
+__device__ __forceinline__ void record_retry(const CellLaunch &a, int sid, int need, int ntri) {
+  AheadRecord r;
+  r.need = (unsigned short)need;
+  for (int k = 0; k < kAheadLevels; ++k) r.jP[k] = r.jV[k] = 255;
+  r.ntri = (unsigned short)ntri;
+  a.ahead[sid] = r;
+}
+
 // Domain restriction of the clipped cell (ConvexCell.cl:918-1116): start
 // corner, boundary triangles, signed cone decomposition.  Adds the cell's
-// moments to acc; returns the status.
+// moments to acc; returns the status.  need: in a retry pass that records
+// (CellLaunch::retry) the neighbours the cell took, else 0.
 template <int VS, bool INL>
 __device__ int restrict_to_domain(WarpCell &w, const CellLaunch &a, const Layout &L, float4 s, int sid_of_cell,
-                                  double acc[4], int lane, unsigned long long *ctr, double *tr, int trcap) {
+                                  double acc[4], int lane, unsigned long long *ctr, double *tr, int trcap,
+                                  int need = 0) {
   const DevGrid &g = a.grid;
   // bounding box -> voxel range (ConvexCell.cl:924-940)
   double lo[3] = {1000.0, 1000.0, 1000.0}, hi[3] = {0.0, 0.0, 0.0};
@@ -2158,6 +2170,7 @@ __device__ int restrict_to_domain(WarpCell &w, const CellLaunch &a, const Layout
   const int S = g.size;
   const int ex = vmax[0] - vmin[0] + 1, ey = vmax[1] - vmin[1] + 1, ez = vmax[2] - vmin[2] + 1;
   const int nvox = (ex > 0 && ey > 0 && ez > 0) ? ex * ey * ez : 0;
+  const bool late = need > a.K;  // a later pass's cell
   bool ahead = false;
   if (g.tsat && nvox > 0) {
     // disjoint lists: the range's triangle count from the summed counts
@@ -2179,10 +2192,11 @@ __device__ int restrict_to_domain(WarpCell &w, const CellLaunch &a, const Layout
       // same cell and restrict it with a larger T; within T_ahead it is
       // parked now, its ids gathered straight into its slot
       if (INL || count > a.T_ahead || !a.defer.slots) {
-        if (a.tri_count && lane == 0) a.tri_count[sid_of_cell] = count;
+        if (a.tri_count && lane == 0 && !late) a.tri_count[sid_of_cell] = count;
         return kTriangleOverflow;
       }
       ahead = true;
+      if ((late || count > a.T_sure) && lane == 0) record_retry(a, sid_of_cell, need, count);
     }
   }
   const DeferQueue &dq = a.defer;
@@ -2323,6 +2337,7 @@ __device__ int restrict_to_domain(WarpCell &w, const CellLaunch &a, const Layout
     park_fixed(dq, slot, a.diag, sid_of_cell, kTriangleOverflow, lane);
     return kDeferred;
   }
+  if (late && !inner && nuniq > 0) return kSecurityRadiusNotReached;
   if (!ahead && dq.slots && (!INL || nuniq > dq.inline_max)) {
     if (lane == 0) slot = atomicAdd(&dq.counters[0], 1);
     slot = __shfl_sync(kFull, slot, 0);
@@ -2333,7 +2348,7 @@ __device__ int restrict_to_domain(WarpCell &w, const CellLaunch &a, const Layout
     // park the cell: its triangles become work items of k_cone
     park_cell(w, dq, slot, L, a.diag, sid_of_cell, nuniq, inner, acc, lane, ahead);
     // the retry passes' T schedule follows the counts settled ahead
-    if (ahead && lane == 0) atomicMax(a.ahead_max ? a.ahead_max : &dq.counters[3], ntr);
+    if (ahead && lane == 0 && !late && ntr <= a.T_sure) atomicMax(a.ahead_max ? a.ahead_max : &dq.counters[3], ntr);
     return kDeferred;
   }
   if constexpr (!INL) {
@@ -2521,14 +2536,14 @@ __device__ __forceinline__ int vertex_capacity(const CellLaunch &a, const Layout
 // Hessian row, used marks); outside: proven outside the domain, mass 0.
 template <int VS, bool GRID, bool INL>
 __device__ __forceinline__ void finish_cell(WarpCell &w, const CellLaunch &a, const Layout &L, float4 s, int sid,
-                                            int status, bool outside, int lane, double *tr, int trcap) {
+                                            int status, bool outside, int lane, double *tr, int trcap, int need = 0) {
   const int np_cell = w.np;  // the clipped cell's planes (cone planes come after)
   double acc[4] = {0, 0, 0, 0};
   unsigned long long *ctr = a.counters;
   if (outside) count(ctr, kCtrOutside, 1, lane);
   if (status == kSuccess && !outside) {
     if (GRID)
-      status = restrict_to_domain<VS, INL>(w, a, L, s, sid, acc, lane, ctr, tr, trcap);
+      status = restrict_to_domain<VS, INL>(w, a, L, s, sid, acc, lane, ctr, tr, trcap, need);
     else
       integrate<VS, INL>(w, 1.0, acc, lane, ctr, tr, trcap);
   }
@@ -2594,7 +2609,7 @@ __device__ __forceinline__ bool settle_ahead(const CellLaunch &a, int sid, bool 
   }
   const AheadRecord r = a.ahead[sid];
   if (r.need == 0) return false;
-  if (lead) a.status[sid] = ahead_status(r, a.K, a.lP, a.lV);
+  if (lead) a.status[sid] = ahead_status(r, a.K, a.T, a.lP, a.lV);
   return true;
 }
 
@@ -2612,6 +2627,7 @@ __device__ __forceinline__ void cell_row(const CellLaunch &a, const Layout &L, u
   unsigned long long *ctr = a.counters;
   const int sid = a.ids ? a.ids[row] : row;
   if (only_status >= 0 && a.status[sid] != only_status) return;
+  if (a.retry && lane == 0) a.ahead[sid].need = 0;
   // Hessian rows run inline only (no defer queue)
   if constexpr (INL) {
     if (a.hess && lane == 0) a.hessid[size_t(sid) * a.H] = -1;  // an empty row until the cell succeeds
@@ -2630,7 +2646,7 @@ __device__ __forceinline__ void cell_row(const CellLaunch &a, const Layout &L, u
       }
     }
   }
-  if (a.ahead && settle_ahead(a, sid, lane == 0)) return;
+  if (a.ahead && !a.retry && settle_ahead(a, sid, lane == 0)) return;
   const float4 s = a.stored[sid];
   double *tr = (a.trace && sid == a.trace_seed) ? a.trace : nullptr;
   const int trcap = a.trace_cap;
@@ -2663,6 +2679,8 @@ __device__ __forceinline__ void cell_row(const CellLaunch &a, const Layout &L, u
 
   // ---- power clipping by the K nearest, in order ----
   const unsigned *nrow = a.knn + size_t(row) * a.Kx;
+  const int Kend = a.retry ? a.Kx : a.K;
+  int last = 0;  // the neighbour that ended the clipping
   bool reached = false, exhausted = false, outside = false;
   const bool early = GRID && a.early_out && a.grid.sat != nullptr && a.wmin != nullptr && a.border_d == 0;
   double plain2 = early ? plain_radius2(a.grid, s, lane) : -1.0;
@@ -2679,14 +2697,14 @@ __device__ __forceinline__ void cell_row(const CellLaunch &a, const Layout &L, u
       return -1.0;
     }
   };
-  for (int i0 = 0; i0 < a.K && status == kSuccess && !reached && !exhausted && !outside; i0 += 32) {
+  for (int i0 = 0; i0 < Kend && status == kSuccess && !reached && !exhausted && !outside; i0 += 32) {
     // every lane builds the bisector of one neighbour, in double
     const int i = i0 + lane;
     Plane pl{0.0, 0.0, 0.0, 0.0};
     double nd2 = 0.0;
     bool valid = false;
     unsigned zl = kNone;
-    if (i < a.K) {
+    if (i < Kend) {
       const unsigned z = __ldg(&nrow[i]);
       zl = z;
       if (z != kNone) {
@@ -2698,8 +2716,9 @@ __device__ __forceinline__ void cell_row(const CellLaunch &a, const Layout &L, u
     const float4 pl32 = PREC ? plane_f(pl) : make_float4(0.f, 0.f, 0.f, 0.f);
     const unsigned vmask = __ballot_sync(kFull, valid);
     if (i0 == 0 && plain2 >= 0.0 && !nonempty_cell(s, vmask, __shfl_sync(kFull, nd2, 0), a.wmin)) plain2 = -1.0;
-    const int cnt = min(32, a.K - i0);
+    const int cnt = min(32, Kend - i0);
     for (int j = 0; j < cnt; ++j) {
+      last = i0 + j;
       if (!((vmask >> j) & 1u)) {
         exhausted = true;  // fewer than K other seeds: all have been clipped
         break;
@@ -2729,7 +2748,7 @@ __device__ __forceinline__ void cell_row(const CellLaunch &a, const Layout &L, u
           R2 = cell_radius2<VS>(w, lane);
           if (R2 <= plain2) {
             out_known = true;
-            if (outside_certain<VS, PREC>(w, a, nrow, s, i0, i0 + j, pl, nd2, valid, R2, safe_dw(), lane)) {
+            if (last < a.K && outside_certain<VS, PREC>(w, a, nrow, s, i0, i0 + j, pl, nd2, valid, R2, safe_dw(), lane)) {
               outside = true;
               break;
             }
@@ -2756,7 +2775,7 @@ __device__ __forceinline__ void cell_row(const CellLaunch &a, const Layout &L, u
             }
             if (out) {
               out_known = true;
-              if (outside_certain<VS, PREC>(w, a, nrow, s, i0, i0 + j, pl, nd2, valid,
+              if (last < a.K && outside_certain<VS, PREC>(w, a, nrow, s, i0, i0 + j, pl, nd2, valid,
                                             R2 >= 0.0 ? R2 : double(R2hi), safe_dw(), lane)) {
                 outside = true;
                 break;
@@ -2801,7 +2820,11 @@ __device__ __forceinline__ void cell_row(const CellLaunch &a, const Layout &L, u
     if (status == kSuccess && !outside && a.border_d == 0) promote(w, lane);
   }
   if (status == kSuccess && !reached && !exhausted && !outside) status = kSecurityRadiusNotReached;
+  if (last >= a.K && status != kSuccess) status = kSecurityRadiusNotReached;  // fails so in this pass
   if (status == kSuccess && out_known) outside = true;
+  // (outside: the radius is surely reached with K)
+  const int need = !a.retry ? 0 : last + 1;
+  if (need > a.K && status == kSuccess && lane == 0) record_retry(a, sid, need, 0);
   if (a.border_d > 0) {
     // bordering pass (ConvexCell.cl:756-809): the clipped cell marks its
     // neighbours; statuses and moments stay those of the main passes
@@ -2809,7 +2832,7 @@ __device__ __forceinline__ void cell_row(const CellLaunch &a, const Layout &L, u
     if (status == kSuccess) mark_neighbours(a.used, w.tri, w.nv, w.pnb, a.border_d, lane, 32);
     return;
   }
-  finish_cell<VS, GRID, INL>(w, a, L, s, sid, status, outside, lane, tr, trcap);
+  finish_cell<VS, GRID, INL>(w, a, L, s, sid, status, outside, lane, tr, trcap, need);
 }
 
 template <int VS, bool GRID, bool INL, int PREC = 0, int SAFE = 0>

@@ -447,7 +447,7 @@ __device__ __noinline__ void oct_finish(const CellLaunch &a, const OctLayout &L,
         r.jP[k] = oc.jP[k];
         r.jV[k] = oc.jV[k];
       }
-      r.pad = 0;
+      r.ntri = 0;
       a.ahead[sid] = r;
     }
   }

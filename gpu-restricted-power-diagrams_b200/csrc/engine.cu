@@ -103,13 +103,16 @@ __global__ void k_fail_flags(const int *__restrict__ ids, int num, const int *__
 }
 
 // Settles the listed cells that have a record (CellLaunch::ahead) in a pass of
-// K neighbours and cap levels lP and lV; the others go to `out`, *count of
-// them (zeroed before), every warp's in order.  Bound by memory latency; it
+// K neighbours, T triangles and cap levels lP and lV; the others go to `out`,
+// *count of them (zeroed before, with count[1]), every warp's in order.
+// Triangle overflows of up to T_sure are settled ahead as the pass's kernels
+// would; count[1]: the largest such count.  Bound by memory latency; it
 // takes the settled rows out of the passes' kernels, which ran mostly empty
 // octets: 2M blue-noise seeds' passes 2 and 3 with the neighbour search
 // 12.8 -> 8.5 ms.
-__global__ void k_settle_ahead(const int *__restrict__ ids, int num, const AheadRecord *__restrict__ rec, int K, int lP,
-                               int lV, int *__restrict__ status, int *__restrict__ out, int *__restrict__ count) {
+__global__ void k_settle_ahead(const int *__restrict__ ids, int num, const AheadRecord *__restrict__ rec, int K, int T,
+                               int T_sure, int lP, int lV, int *__restrict__ status, int *__restrict__ out,
+                               int *__restrict__ count) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
   bool left = false;
   int sid = 0;
@@ -117,7 +120,11 @@ __global__ void k_settle_ahead(const int *__restrict__ ids, int num, const Ahead
     sid = ids[i];
     const AheadRecord r = rec[sid];
     left = r.need == 0;
-    if (!left) status[sid] = ahead_status(r, K, lP, lV);
+    if (!left) {
+      const int st = ahead_status(r, K, max(T, T_sure), lP, lV);
+      status[sid] = st;
+      if (st == kSuccess && r.ntri > T) atomicMax(&count[1], int(r.ntri));
+    }
   }
   const unsigned m = __ballot_sync(kFull, left);
   int base = 0;
@@ -130,6 +137,87 @@ __global__ void k_clear_failed(const int *__restrict__ ids, int num, const int *
                                double4 *__restrict__ out) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < num && status[ids[i]] != kSuccess) out[ids[i]] = make_double4(0.0, 0.0, 0.0, 0.0);
+}
+
+// After a retry pass with records (CellLaunch::retry): a recorded cell that
+// went well gets this pass's status, any other failed as this pass's does and
+// loses its record.
+__global__ void k_retry_status(const int *__restrict__ ids, int num, AheadRecord *__restrict__ rec, int K, int T, int lP,
+                               int lV, int *__restrict__ status) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= num) return;
+  const int sid = ids[i];
+  const AheadRecord r = rec[sid];
+  if (r.need == 0) return;
+  if (status[sid] != kSuccess) rec[sid].need = 0;
+  status[sid] = ahead_status(r, K, T, lP, lV);
+}
+
+// The failing lists of few cells in one block and one launch: first the
+// recorded ones of `rows` settled (rec; as k_settle_ahead), then
+// recompute_ids' lists and histogram of ids (null: 0 .. num - 1).  res (16):
+// the histogram, [12] and [13] the lists' lengths, [14] the rows left, [15]
+// k_settle_ahead's count[1].  Bound by latency (a few us); the general path is nine launches.
+constexpr int kSmallList = 4096;
+__global__ void __launch_bounds__(1024) k_small_lists(const int *__restrict__ ids, int num, int *__restrict__ status,
+                                                      int cond, int *out0, int *out1,
+                                                      int *__restrict__ res, const AheadRecord *__restrict__ rec,
+                                                      const int *rows, int nrows, int K, int T, int T_sure, int lP,
+                                                      int lV, int *__restrict__ left) {
+  __shared__ int hist[16], part[32], tmax;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  if (t < 16) hist[t] = 0;
+  if (t == 16) tmax = 0;
+  __syncthreads();
+  // appends v of the threads with f to out + base in order; the new base
+  auto append = [&](bool f, int v, int *out, int base) {
+    const unsigned m = __ballot_sync(kFull, f);
+    if (lane == 0) part[warp] = __popc(m);
+    __syncthreads();
+    const int c = part[lane];
+    int incl = c;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(kFull, incl, o);
+      if (lane >= o) incl += y;
+    }
+    const int before = __shfl_sync(kFull, incl - c, warp), total = __shfl_sync(kFull, incl, 31);
+    if (f) out[base + before + __popc(m & ((1u << lane) - 1u))] = v;
+    __syncthreads();
+    return base + total;
+  };
+  int nleft = 0;
+  if (rec) {
+    for (int b = 0; b < nrows; b += 1024) {
+      const int sid = b + t < nrows ? rows[b + t] : -1;
+      bool f = false;
+      if (sid >= 0) {
+        const AheadRecord r = rec[sid];
+        f = r.need == 0;
+        if (!f) {
+          const int st = ahead_status(r, K, max(T, T_sure), lP, lV);
+          status[sid] = st;
+          if (st == kSuccess && r.ntri > T) atomicMax(&tmax, int(r.ntri));
+        }
+      }
+      nleft = append(f, sid, left, nleft);
+    }
+  }
+  int n0 = 0, n1 = 0;
+  if (nleft == 0) {  // rows are no longer needed: out1 may be their list
+    for (int b = 0; b < num; b += 1024) {
+      int sid = -1, st = kSuccess;
+      if (b + t < num) {
+        sid = ids ? ids[b + t] : b + t;
+        st = status[sid];
+      }
+      if (st != kSuccess) atomicAdd(&hist[st], 1);
+      n0 = append(st != kSuccess, sid, out0, n0);
+      n1 = append(st != kSuccess && (cond == 0 || st != kEmptyCell), sid, out1, n1);
+    }
+  }
+  __syncthreads();
+  if (t < 16) res[t] = t == 12 ? n0 : t == 13 ? n1 : t == 14 ? nleft : t == 15 ? tmax : hist[t];
 }
 
 __global__ void k_fail_scatter(const int *__restrict__ ids, int num, const int *__restrict__ f0,
@@ -293,11 +381,41 @@ namespace {
 // Failing ids of the cells in `ids_in` (null: all n) into out0 (all
 // failing) and out1 (failing, filtered by cond), their counts and the status
 // histogram; synchronous.
+//
+// Of few cells (kSmallList: one block's work) with one launch; then `settle`
+// (optional) first settles the recorded cells of its rows in a pass of its
+// caps, and with rows left (nleft, ids in fail_ws) computes nothing else.
+struct Settle {
+  const int *rows;
+  int nrows, K, T, T_sure, nleft, tmax;
+};
+
 int recompute_ids(rpd_solver *s, const int *ids_in, int num, int cond, int *out0, int *out1, int &n0, int &n1,
-                  int hist[kStatusNum]) {
+                  int hist[kStatusNum], Settle *settle = nullptr) {
   rpd_context *ctx = s->ctx;
   cudaStream_t st = ctx->stream;
   cudaError_t e;
+  if (num <= kSmallList) {
+    if ((e = s->fail_ws.ensure(sizeof(int) * kSmallList)) != cudaSuccess) return map_cuda(ctx, e, "alloc fail ws");
+    int *h = s->hist.as<int>();
+    k_small_lists<<<1, 1024, 0, st>>>(ids_in, num, s->status.as<int>(), cond, out0, out1, h,
+                                      settle ? s->ahead.as<AheadRecord>() : nullptr, settle ? settle->rows : nullptr,
+                                      settle ? settle->nrows : 0, settle ? settle->K : 0, settle ? settle->T : 0,
+                                      settle ? settle->T_sure : 0, s->level_P, s->level_V, s->fail_ws.as<int>());
+    s->stats.kernel_launches += 1;
+    int hh[16];
+    if ((e = cudaMemcpyAsync(hh, h, sizeof(hh), cudaMemcpyDeviceToHost, st)) != cudaSuccess)
+      return map_cuda(ctx, e, "copy hist");
+    if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return map_cuda(ctx, e, "recompute ids");
+    if (settle) {
+      settle->tmax = hh[15];
+      if ((settle->nleft = hh[14]) > 0) return RPD_OK;
+    }
+    for (int i = 0; i < kStatusNum; ++i) hist[i] = hh[i];
+    n0 = hh[12];
+    n1 = hh[13];
+    return RPD_OK;
+  }
   const size_t nsc = scan_workspace_ints(num + 1);
   if ((e = s->fail_ws.ensure(sizeof(int) * (4 * size_t(num + 1) + nsc))) != cudaSuccess)
     return map_cuda(ctx, e, "alloc fail ws");
@@ -470,7 +588,8 @@ constexpr int kOctetMinRows = 4096;
 static_assert(int(RPD_CTR_NUM) == int(kCtrNum), "counter enums out of sync");
 
 int run_pass(rpd_solver *s, const int *ids, int num, int K, int P, int V, int T, float eps, int out_domain,
-             bool counters, bool early_out, int border_d = 0, int T_ahead = 0, int out_domain_ahead = 0) {
+             bool counters, bool early_out, int border_d = 0, int T_ahead = 0, int out_domain_ahead = 0,
+             int retry_K = 0, int T_sure = kMaxT) {
   rpd_context *ctx = s->ctx;
   cudaStream_t st = ctx->stream;
   cudaError_t e;
@@ -481,7 +600,7 @@ int run_pass(rpd_solver *s, const int *ids, int num, int K, int P, int V, int T,
   const bool all_cells = ids == nullptr && num == s->n;
   rpd::DevBuf &kb = all_cells ? s->knn : s->knn_part;
   const bool ahead_first = s->ahead_on && pi == 0;
-  const int Kx = ahead_first ? ahead_columns(K) : K;
+  const int Kx = ahead_first ? ahead_columns(K) : retry_K > 0 ? retry_K : K;
   const bool reuse = all_cells && s->knn_full_K == K && s->knn_full_Kx == Kx && !counters && !s->fresh_knn;
   if ((e = kb.ensure(sizeof(unsigned) * size_t(num) * Kx)) != cudaSuccess) return map_cuda(ctx, e, "alloc knn");
   Events<4> ev;
@@ -577,6 +696,11 @@ int run_pass(rpd_solver *s, const int *ids, int num, int K, int P, int V, int T,
       a.ladV[k] = s->lad_V[k];
     }
   }
+  if (retry_K > 0) {
+    a.ahead = s->ahead.as<AheadRecord>();
+    a.retry = 1;
+    a.T_sure = T_sure;
+  }
   if (num >= kOctetMinRows && octet_applies(a)) {
     ClipHand &hd = a.hand;
     hd.capacity = clip_hand_capacity(num);
@@ -607,6 +731,10 @@ int run_pass(rpd_solver *s, const int *ids, int num, int K, int P, int V, int T,
       b.after_cell = nullptr;
       if ((e = cell_launch(b, st, ctx->sm_count, &launches)) != cudaSuccess) return map_cuda(ctx, e, "cell kernel");
     }
+  }
+  if (a.retry && num > 0) {
+    k_retry_status<<<(num + 255) / 256, 256, 0, st>>>(ids, num, a.ahead, K, std::max(T, T_sure), s->level_P, s->level_V, a.status);
+    launches += 1;
   }
   S.kernel_launches += launches - 1;
   cudaEventRecord(ev[2], st);
@@ -1141,12 +1269,12 @@ static int launch_impl(rpd_solver *s, const rpd_params *pp, const PartSpec *part
   }
   // cells clipped past the first pass's caps, so that the retries can settle
   // them from a record (tight caps fail most cells)
-  s->ahead_on = ahead_pays(p.K, p.V) && !counters && !s->used_on && s->hess_h == 0 && !(p.flags & RPD_FLAG_SAFE_RADIUS) &&
-                s->precision <= 1 && p.max_extra_passes > 0 && !(p.flags & RPD_FLAG_FIRST_PASS_ONLY) &&
-                count >= kOctetMinRows;
+  const bool retries_ok = !counters && !s->used_on && s->hess_h == 0 && !(p.flags & RPD_FLAG_SAFE_RADIUS) &&
+                          s->precision <= 1 && p.max_extra_passes > 0 && !(p.flags & RPD_FLAG_FIRST_PASS_ONLY);
+  s->ahead_on = retries_ok && ahead_pays(p.K, p.V) && count >= kOctetMinRows;
+  s->level_P = s->level_V = 0;
   if (s->ahead_on) {
     if ((e = s->ahead.ensure(sizeof(AheadRecord) * size_t(n))) != cudaSuccess) return map_cuda(ctx, e, "alloc records");
-    s->level_P = s->level_V = 0;
     for (int k = 0, P = p.P, V = p.V; k < kAheadLevels; ++k, P = int(P * 1.5), V = std::min(int(V * 1.5), kMaxV)) {
       s->lad_P[k] = P;
       s->lad_V[k] = V;
@@ -1165,6 +1293,7 @@ static int launch_impl(rpd_solver *s, const rpd_params *pp, const PartSpec *part
   int K = p.K, P = p.P, V = p.V, T = p.T;
   if (!(p.flags & RPD_FLAG_FIRST_PASS_ONLY)) {
     int hist[kStatusNum];
+    bool live = s->ahead_on;  // cells have records
     int n0 = 0, n1 = 0, n0_all = 0;  // n0: this part's failing cells; n0_all: every part's
     int *A = s->ids_a.as<int>(), *B = s->ids_b.as<int>(), *Cc = s->ids_c.as<int>();
     // extra passes (voronoi.cpp:1311-1376): caps grow x1.5 by failing status
@@ -1188,21 +1317,67 @@ static int launch_impl(rpd_solver *s, const rpd_params *pp, const PartSpec *part
       const int T_later = T_ahead > 0 ? t_ahead_cap(P, K, T, p.max_extra_passes - step - 1) : 0;
       const int *rows = Cc;
       int nrows = n1;
-      if (s->ahead_on && n1 > 0) {
+      const int pi = s->stats.npasses;
+      if (live && n1 > 0) {
         // recorded cells are settled here, the others (fail_ws holds their
         // ids until the next recompute_ids) solved again
-        int *left = s->fail_ws.as<int>(), *count = s->hist.as<int>() + 15;
-        cudaMemsetAsync(count, 0, sizeof(int), st);
-        k_settle_ahead<<<(n1 + 255) / 256, 256, 0, st>>>(Cc, n1, s->ahead.as<AheadRecord>(), K, s->level_P, s->level_V,
-                                                        s->status.as<int>(), left, count);
-        s->stats.kernel_launches += 1;
-        if ((e = cudaMemcpyAsync(&nrows, count, sizeof(int), cudaMemcpyDeviceToHost, st)) != cudaSuccess ||
-            (e = cudaStreamSynchronize(st)) != cudaSuccess)
-          return map_cuda(ctx, e, "settle ahead");
+        int *left = s->fail_ws.as<int>(), *count = s->hist.as<int>() + 14;
+        if (n0 <= kSmallList) {
+          Settle z{Cc, n1, K, T, T_later, 0, 0};
+          const int rows_n = n1;
+          if ((rc = recompute_ids(s, A, n0, 1, B, Cc, n0, n1, hist, &z)) != RPD_OK) return rc;
+          nrows = z.nleft;
+          s->ahead_max = std::max(s->ahead_max, z.tmax);
+          if (nrows == 0) {  // a pass without work
+            if (pi < 8) {
+              s->stats.pass_cells[pi] = rows_n;
+              s->stats.pass_K[pi] = K;
+              s->stats.pass_P[pi] = P;
+              s->stats.pass_V[pi] = V;
+              s->stats.pass_T[pi] = T;
+            }
+            s->stats.npasses++;
+            std::swap(A, B);
+            n0_all = n0;
+            if ((rc = reduce_schedule(s, part, hist, n0_all)) != RPD_OK) return rc;
+            continue;
+          }
+        } else {
+          int got[2];
+          cudaMemsetAsync(count, 0, sizeof(got), st);
+          k_settle_ahead<<<(n1 + 255) / 256, 256, 0, st>>>(Cc, n1, s->ahead.as<AheadRecord>(), K, T, T_later, s->level_P,
+                                                          s->level_V, s->status.as<int>(), left, count);
+          s->stats.kernel_launches += 1;
+          if ((e = cudaMemcpyAsync(got, count, sizeof(got), cudaMemcpyDeviceToHost, st)) != cudaSuccess ||
+              (e = cudaStreamSynchronize(st)) != cudaSuccess)
+            return map_cuda(ctx, e, "settle ahead");
+          nrows = got[0];
+          s->ahead_max = std::max(s->ahead_max, got[1]);
+        }
         rows = left;
       }
-      const int pi = s->stats.npasses;
-      if ((rc = run_pass(s, rows, nrows, K, P, V, T, eps, out_domain, counters, early, 0, T_later, out_domain)) != RPD_OK)
+      // few cells: clipped with the next pass's K too and restricted up to
+      // the last pass's T, their statuses in those passes then known.  A pass
+      // of few cells takes 0.2 to 0.5 ms however few (one warp's latency, the
+      // cones', three waits of the host), so passes saved count: 1K seeds
+      // 1.07 -> 0.82 ms, 30K in the box 1.30 -> 1.08, 100K in a blob 4.33 ->
+      // 3.66, 50K in a field 3.82 -> 3.08.  Two or four levels of K take
+      // longer for the neighbours (0.02 to 0.1 ms) and save no pass more.
+      // From kOctetMinRows on a pass's time is its cells', which the longer
+      // rows would cost.
+      int retry_K = 0, T_most = T_later;
+      const int rest = p.max_extra_passes - step - 1;
+      if (retries_ok && nrows > 0 && nrows < kOctetMinRows && rest > 0) {
+        retry_K = K;
+        if (int(K * 1.5) <= kMaxK) retry_K = int(K * 1.5);
+        if (T_ahead > 0)
+          for (int j = 0, t = T; j < rest; ++j) T_most = t = std::min(int(t * 1.5), kMaxT);
+        if ((e = s->ahead.ensure(sizeof(AheadRecord) * size_t(n))) != cudaSuccess)
+          return map_cuda(ctx, e, "alloc records");
+        live = true;
+      }
+      if ((rc = run_pass(s, rows, nrows, K, P, V, T, eps, out_domain, counters, early, 0, T_most, out_domain, retry_K,
+                         T_later)) != RPD_OK)
         return rc;
       if (pi < 8) s->stats.pass_cells[pi] = n1;  // the reference solves all of them again
       if ((rc = recompute_ids(s, A, n0, 1, B, Cc, n0, n1, hist)) != RPD_OK) return rc;
@@ -1210,7 +1385,7 @@ static int launch_impl(rpd_solver *s, const rpd_params *pp, const PartSpec *part
       n0_all = n0;
       if ((rc = reduce_schedule(s, part, hist, n0_all)) != RPD_OK) return rc;
     }
-    if (s->ahead_on && n0 > 0) {
+    if (live && n0 > 0) {
       // the recorded cells that no pass settled: failed, no moments
       k_clear_failed<<<(n0 + 255) / 256, 256, 0, st>>>(A, n0, s->status.as<int>(), s->out.as<double4>());
       s->stats.kernel_launches += 1;
