@@ -5,7 +5,9 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <map>
 #include <mutex>
+#include <new>
 #include <string>
 
 #include "engine.cuh"
@@ -17,10 +19,24 @@ constexpr int kMaxDev = 64;
 std::mutex g_alloc_mu;
 cudaStream_t g_alloc_stream[kMaxDev] = {};
 
-cudaError_t alloc_stream(cudaStream_t *out) {
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
+// Freed blocks by size class (never destroyed: buffers may outlive statics).
+struct Kept {
+  std::mutex mu;
+  std::map<size_t, std::vector<void *>> blocks;
+  size_t bytes = 0;
+  int contexts = 0;
+};
+Kept *const g_kept = new Kept[kMaxDev];
+constexpr size_t kKeepBlock = size_t(1) << 30, kKeepBytes = size_t(8) << 30;
+
+size_t size_class(size_t bytes) {
+  size_t step = 512;
+  while (step * 16 <= bytes) step *= 2;
+  return (bytes + step - 1) / step * step;
+}
+
+cudaError_t alloc_stream(int dev, cudaStream_t *out) {
+  cudaError_t e;
   if (dev < 0 || dev >= kMaxDev) return cudaErrorInvalidDevice;
   std::lock_guard<std::mutex> lock(g_alloc_mu);
   if (!g_alloc_stream[dev]) {
@@ -37,20 +53,75 @@ cudaError_t alloc_stream(cudaStream_t *out) {
 }
 }  // namespace pool_detail
 
-cudaError_t pool_alloc(void **p, size_t bytes) {
+// Returns the kept blocks of a device to the driver's pool.
+static void pool_flush(int dev) {
+  using namespace pool_detail;
   cudaStream_t st;
-  cudaError_t e = pool_detail::alloc_stream(&st);
+  if (alloc_stream(dev, &st) != cudaSuccess) return;
+  std::lock_guard<std::mutex> lock(g_kept[dev].mu);
+  for (auto &c : g_kept[dev].blocks)
+    for (void *p : c.second) cudaFreeAsync(p, st);
+  g_kept[dev].blocks.clear();
+  g_kept[dev].bytes = 0;
+}
+
+cudaError_t pool_alloc(void **p, size_t bytes, int *device) {
+  using namespace pool_detail;
+  int dev = 0;
+  cudaStream_t st;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess || (e = alloc_stream(dev, &st)) != cudaSuccess) return e;
+  *device = dev;
+  if (bytes <= kKeepBlock) {
+    bytes = size_class(bytes);
+    std::lock_guard<std::mutex> lock(g_kept[dev].mu);
+    auto c = g_kept[dev].blocks.find(bytes);
+    if (c != g_kept[dev].blocks.end() && !c->second.empty()) {
+      *p = c->second.back();
+      c->second.pop_back();
+      g_kept[dev].bytes -= bytes;
+      return cudaSuccess;
+    }
+  }
+  if ((e = cudaMallocAsync(p, bytes, st)) == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    pool_flush(dev);
+    e = cudaMallocAsync(p, bytes, st);
+  }
   if (e != cudaSuccess) return e;
-  if ((e = cudaMallocAsync(p, bytes, st)) != cudaSuccess) return e;
   // usable from every stream once the allocation stream has reached it
   return cudaStreamSynchronize(st);
 }
 
-void pool_free(void *p) {
+void pool_free(void *p, size_t bytes, int dev) {
+  using namespace pool_detail;
+  if (bytes <= kKeepBlock) {
+    bytes = size_class(bytes);
+    std::lock_guard<std::mutex> lock(g_kept[dev].mu);
+    if (g_kept[dev].contexts > 0 && g_kept[dev].bytes + bytes <= kKeepBytes) {
+      try {
+        g_kept[dev].blocks[bytes].push_back(p);
+        g_kept[dev].bytes += bytes;
+        return;
+      } catch (const std::bad_alloc &) {  // then to the driver's pool
+      }
+    }
+  }
   cudaStream_t st;
-  if (pool_detail::alloc_stream(&st) == cudaSuccess) cudaFreeAsync(p, st);
+  if (alloc_stream(dev, &st) == cudaSuccess) cudaFreeAsync(p, st);
 }
 
+void pool_context(int dev, int change) {
+  using namespace pool_detail;
+  if (dev < 0 || dev >= kMaxDev) return;
+  bool last;
+  {
+    std::lock_guard<std::mutex> lock(g_kept[dev].mu);
+    g_kept[dev].contexts += change;
+    last = g_kept[dev].contexts <= 0;
+  }
+  if (last) pool_flush(dev);
+}
 
 namespace {
 thread_local std::string g_cuda_error;
@@ -784,6 +855,7 @@ rpd_context *rpd_context_create(int device, int *err) {
     if (err) *err = RPD_ERR_CUDA;
     return nullptr;
   }
+  pool_context(device, 1);
   if (err) *err = RPD_OK;
   return ctx;
 }
@@ -795,7 +867,9 @@ void rpd_context_destroy(rpd_context *ctx) {
     cudaStreamSynchronize(ctx->stream);
     cudaStreamDestroy(ctx->stream);
   }
+  const int device = ctx->device;
   delete ctx;
+  pool_context(device, -1);
 }
 
 const char *rpd_context_error(const rpd_context *ctx) { return ctx ? ctx->error.c_str() : ""; }
