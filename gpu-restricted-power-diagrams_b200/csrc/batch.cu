@@ -809,8 +809,8 @@ int capture(rpd_batch *b) {
   int launches = 0;
   // The first pass's neighbour-search variant per slot class (the
   // autotuner): the probe and the first pass's plan run once outside the
-  // graph, so the records and rows exist, then each class large enough to
-  // tell (16K rows) is searched both ways on its own rows, timed with events
+  // graph, so the records and rows exist, then a class of K <= 32 large
+  // enough to tell (16K rows) is searched both ways on its own rows, timed with events
   // (one untimed round first); the graph takes the faster.  Retry passes
   // (few rows) take a warp per seed.
   int variant[kKnnClasses];

@@ -46,8 +46,12 @@ enum CellCounter {
 };
 
 // Triangles of one work item of the cone kernels; a cell's sum adds its
-// chunks' sums in order, also where a cell's own warp takes them all.
-constexpr int kConeChunk = 16;
+// chunks' sums in order, also where a cell's own warp takes them all.  A warp
+// takes four triangles at a time, about 30 us each time: a pass of few cells
+// lasts as long as one item.  16 -> 8: 1K seeds 0.82 -> 0.65 ms, 100K in a
+// blob 3.65 -> 3.39, 50K in a field 3.08 -> 2.84, 1M 11.8 -> 11.7; 48 uneven
+// diagrams 60.6 -> 61.2 (more items load and prepare their cell).
+constexpr int kConeChunk = 8;
 
 // Boundary cells with many triangles park their clipped cell here; a second
 // kernel spreads their triangles over all warps in chunks.

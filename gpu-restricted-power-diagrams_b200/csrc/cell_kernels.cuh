@@ -1519,7 +1519,7 @@ __device__ int drop_separated(const WarpCell &w, const DevGrid &g, float4 s, int
 // faces that they cut -- in one list of the warp, whose entries the 32 lanes
 // then take.  One lane per triangle, the form before, kept 10 of 32 lanes
 // busy (the triangles' faces and cuts differ) and took 200 us for one work
-// item, the whole launch of a small diagram; now 18 of 32 and 100 us.  Clip
+// item, the whole launch of a small diagram; now 18 of 32 and 30 us per four.  Clip
 // bounds are compared as fractions, so that a segment costs two divisions
 // and not one per plane.  Measured, cone kernels of the first pass: 250K
 // uniform seeds in a cube 2.5 -> 1.5 ms, 2M blue noise (second pass) 5.6 ->

@@ -1323,7 +1323,7 @@ static int launch_impl(rpd_solver *s, const rpd_params *pp, const PartSpec *part
   // retry pass, which restricts it once T has grown past its count.  The
   // retries certainly run while this cell fails, up to max_extra_passes,
   // unless P or K outgrow their limits; assuming both grow in every pass,
-  // the first pass parks such cells up to the T of the last retry that
+  // every pass parks such cells up to the T of the last retry that
   // surely runs, and restricts them as a retry would
   const int out_domain = p.out_domain >= 0 ? p.out_domain : (grid && s->grid.has_border_corners ? 1 : 0);
   int T_ahead = 0;

@@ -203,10 +203,9 @@ rpd_grid *rpd_solver_export_grid(rpd_solver *s, int *err);
                                          the last launch (same results) */
 #define RPD_FLAG_NO_PROBE 64u       /* no outside probe (the default; overrides
                                        RPD_FLAG_OUTSIDE_PROBE) */
-#define RPD_FLAG_NO_T_AHEAD 128u    /* leave every triangle overflow of the first pass
-                                       to the retry passes instead of restricting at
-                                       once the cells the retries would settle (same
-                                       results) */
+#define RPD_FLAG_NO_T_AHEAD 128u    /* leave every triangle overflow to the retry
+                                       passes instead of restricting at once the cells
+                                       the retries would settle (same results) */
 #define RPD_FLAG_OUTSIDE_PROBE 2048u /* before the first pass, settle the cells that a probe of
                                        their 3x3x3 bins proves outside the domain (mass 0,
                                        status success) without their K-nearest search and
@@ -224,14 +223,15 @@ rpd_grid *rpd_solver_export_grid(rpd_solver *s, int *err);
                                        d_j^2 - 2 R d_j > w_s - min w.  A cell the reference's test
                                        stops early on comes out exact (different from the
                                        reference's); equal weights give the reference's test */
-#define RPD_FLAG_KNN_WARP 256u      /* neighbour search with a warp per seed (bitonic
-                                       merges) for every K (same results) */
+#define RPD_FLAG_KNN_WARP 256u      /* neighbour search with a warp per seed for
+                                       every K (same results) */
 #define RPD_FLAG_KNN_THREAD 512u    /* neighbour search with a thread per seed (a
                                        shared-memory heap) for K <= 128 (same results).
                                        Without either flag, searches of at least 16K
-                                       rows use the variant each context picks for K by
-                                       a timed trial the first time K comes up, smaller
-                                       ones a warp per seed (rpd_stats.pass_knn_variant) */
+                                       rows with K <= 32 use the variant each context
+                                       picks for K by a timed trial the first time K
+                                       comes up, others a warp per seed
+                                       (rpd_stats.pass_knn_variant) */
 
 /* VoroAlgo's knobs (voronoi.h:199-246; defaults of Options.cpp:22-28). */
 typedef struct rpd_params {
@@ -542,8 +542,8 @@ typedef struct rpd_batch_stats {
   long long probe_outside; /* seeds the probe proved empty outside their domains, all diagrams */
   /* The first pass's neighbour search per K class (K <= 32, 64, 96, 128, 192,
    * 256): 0 a warp per seed, 1 a thread per seed, -1 no diagram in the
-   * class; chosen at capture by timing both on the class's own rows (0 ms:
-   * no trial, too few rows or K too large for a thread per seed). */
+   * class; for K <= 32 chosen at capture by timing both on the class's own
+   * rows (0 ms: no trial, too few rows or a larger K, which takes a warp). */
   int knn_variant[6];
   float knn_trial_warp_ms[6], knn_trial_thread_ms[6];
 } rpd_batch_stats;
