@@ -13,6 +13,7 @@ from __future__ import annotations
 import argparse
 import json
 import os
+import select
 import statistics
 import subprocess
 import sys
@@ -98,7 +99,7 @@ MEASURED_FP64_TFLOPS = 34.17
 SMSP_PER_SM = 4  # warp schedulers per SM: one warp instruction each per cycle
 
 
-def profile_counters(config, kernel="k_cell"):
+def profile_counters(config, kernel="k_clip"):
     """The per-launch counters of a committed ncu summary
     (profiles/<kernel>_<config>_counters.txt), or {}."""
     out = {}
@@ -136,8 +137,12 @@ class ClockSampler:
     def start(self):
         try:
             self.proc = subprocess.Popen(
-                ["nvidia-smi", f"--query-gpu={self.FIELDS}", "--format=csv,noheader,nounits", "-lms", "100",
+                ["nvidia-smi", f"--query-gpu={self.FIELDS}", "--format=csv,noheader,nounits", "-lms", "20",
                  "-i", self.index], stdout=subprocess.PIPE, stderr=subprocess.DEVNULL, text=True)
+            # nvidia-smi takes longer to start than ten steps take to run: the
+            # timed region begins once it samples (that line is not counted)
+            if select.select([self.proc.stdout], [], [], 5.0)[0]:
+                self.proc.stdout.readline()
         except Exception:
             self.proc = None
 
@@ -548,7 +553,7 @@ def run_ours(args, cfg, rank, world, local):
     scale = rows / prof["rows"] if prof.get("rows") else None
     sm_mhz = clk.get("sm_mhz") or 1965.0
     issue_peak = 148 * SMSP_PER_SM * sm_mhz * 1e6 / 1e9  # G warp instructions / s
-    roofline = {"kernel": "k_cell (first pass)", "bound": "issue", "unit": "G warp-instructions/s",
+    roofline = {"kernel": "k_clip + k_finish (first pass)", "bound": "issue", "unit": "G warp-instructions/s",
                 "peak": issue_peak, "peak_source": f"148 SMs x {SMSP_PER_SM} schedulers x {sm_mhz:.0f} MHz "
                                                   "(SM clock sampled during the timed steps)",
                 "launch_ms": cell_avg_ms, "rows": rows}
@@ -563,7 +568,7 @@ def run_ours(args, cfg, rank, world, local):
                             "peak": MEASURED_FP64_TFLOPS, "peak_source": "measured (DFMA microbenchmark)",
                             "frac": fp64 / (cell_avg_ms / 1e3) / 1e12 / MEASURED_FP64_TFLOPS,
                             "flops_per_launch": fp64, "work": "executed FP64 instructions (2 DFMA + DADD + DMUL)"}
-        roofline["counters_source"] = f"profiles/k_cell_{args.config}_counters.txt (ncu, one launch)"
+        roofline["counters_source"] = f"profiles/k_clip_{args.config}_counters.txt (ncu, one launch of each)"
     else:
         roofline.update({"achieved": None, "frac": None, "traffic": None,
                          "note": "no committed ncu counters for this workload"})
@@ -762,10 +767,10 @@ def run_batch(args, cfg, rank, world, local):
     # warp instructions per cell from the committed ncu counters of the
     # batch's first 32 diagrams (every cell a row), scaled to this launch
     rows = n - int(bstats.get("probe_outside", 0))
-    prof = profile_counters(args.config, "k_cell_batch")
+    prof = profile_counters(args.config, "k_clip_batch")
     sm_mhz = clk.get("sm_mhz") or 1965.0
     issue_peak = 148 * SMSP_PER_SM * sm_mhz * 1e6 / 1e9
-    roofline = {"kernel": "k_cell_batch (first pass, all diagrams)", "bound": "issue",
+    roofline = {"kernel": "k_clip_batch + k_finish_batch (first pass, all diagrams)", "bound": "issue",
                 "unit": "G warp-instructions/s", "peak": issue_peak,
                 "peak_source": f"148 SMs x {SMSP_PER_SM} schedulers x {sm_mhz:.0f} MHz (SM clock sampled during "
                                "the timed steps)", "launch_ms": cell_avg_ms, "rows": rows,
@@ -782,7 +787,7 @@ def run_batch(args, cfg, rank, world, local):
                                   "frac": fp64 / (cell_avg_ms / 1e3) / 1e12 / MEASURED_FP64_TFLOPS,
                                   "flops_per_launch": fp64,
                                   "work": "executed FP64 instructions (2 DFMA + DADD + DMUL)"},
-                         "counters_source": f"profiles/k_cell_batch_{args.config}_counters.txt (ncu, the first 32 "
+                         "counters_source": f"profiles/k_clip_batch_{args.config}_counters.txt (ncu, the first 32 "
                                             "diagrams' launch, scaled per cell)"})
     else:
         roofline.update({"achieved": None, "frac": None, "traffic": None,
