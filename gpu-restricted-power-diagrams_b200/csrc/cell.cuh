@@ -92,10 +92,11 @@ struct ClipHand {
 // cell from this record instead of clipping it again.
 constexpr int kMaxT = 4096;
 constexpr int kAheadLevels = 6;  // caps of the schedule: the first pass's, grown x1.5 one to five times
+constexpr int kNoStop = 255;     // a level that stops the clipping nowhere (first passes record lists of up to 200)
 struct AheadRecord {
   unsigned short need;  // neighbours it takes to the security radius (0: no record)
-  // the neighbour at which the cap of each level stops the clipping (255: it
-  // does not): before its plane test, and at its cut
+  // the neighbour at which the cap of each level stops the clipping (kNoStop:
+  // none): before its plane test, and at its cut
   unsigned char jP[kAheadLevels], jV[kAheadLevels];
   unsigned short ntri;  // triangles its restriction needs, when more than the T of the recording pass (else 0)
 };
@@ -104,7 +105,9 @@ static_assert(sizeof(AheadRecord) == 16, "ahead record size");
 // The status of a recorded cell in a pass of K neighbours, T triangles and
 // cap levels lP and lV: the first cap that stops it decides.
 __host__ __device__ inline int ahead_status(const AheadRecord &r, int K, int T, int lP, int lV) {
-  const int p = lP < kAheadLevels ? r.jP[lP] : 255, v = lV < kAheadLevels ? r.jV[lV] : 255;
+  const int never = 1 << 16;
+  const int p = lP < kAheadLevels && r.jP[lP] != kNoStop ? r.jP[lP] : never;
+  const int v = lV < kAheadLevels && r.jV[lV] != kNoStop ? r.jV[lV] : never;
   const int first = p < v ? p : v, end = K < r.need ? K : r.need;
   if (first < end) return p <= v ? kPlaneOverflow : kVertexOverflow;
   if (r.need > K) return kSecurityRadiusNotReached;

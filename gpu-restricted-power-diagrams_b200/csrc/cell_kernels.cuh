@@ -2127,7 +2127,7 @@ __device__ void park_fixed(const DeferQueue &dq, int slot, int diag, int sid, in
 __device__ __forceinline__ void record_retry(const CellLaunch &a, int sid, int need, int ntri) {
   AheadRecord r;
   r.need = (unsigned short)need;
-  for (int k = 0; k < kAheadLevels; ++k) r.jP[k] = r.jV[k] = 255;
+  for (int k = 0; k < kAheadLevels; ++k) r.jP[k] = r.jV[k] = kNoStop;
   r.ntri = (unsigned short)ntri;
   a.ahead[sid] = r;
 }

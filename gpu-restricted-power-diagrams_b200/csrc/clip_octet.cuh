@@ -510,7 +510,7 @@ __device__ __forceinline__ void clip_octet(const CellLaunch &a, const OctLayout 
     oc.s = s;
     oc.vst = -1;
     if (ahead) {
-      for (int k = 0; k < kAheadLevels; ++k) oc.jP[k] = oc.jV[k] = 255;
+      for (int k = 0; k < kAheadLevels; ++k) oc.jP[k] = oc.jV[k] = kNoStop;
       oc.lP = oc.lV = 0;
     }
   }
