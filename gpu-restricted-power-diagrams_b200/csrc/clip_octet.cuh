@@ -441,10 +441,13 @@ __device__ __noinline__ void oct_finish(const CellLaunch &a, const OctLayout &L,
     a.status[sid] = ok && vst >= 0 ? vst : status;
     a.out[sid] = ok ? global_moments(acc, s) : make_double4(0.0, 0.0, 0.0, 0.0);
     if (ok && vst >= 0) {
+      // a list that ended at `last` has no neighbour there whose plane test a
+      // cap could stop
+      const bool ended = __ldg(&a.knn[size_t(row) * a.Kx + oc.last]) == kNone;
       AheadRecord r;
       r.need = (unsigned short)(oc.last + 1);
       for (int k = 0; k < kAheadLevels; ++k) {
-        r.jP[k] = oc.jP[k];
+        r.jP[k] = ended && oc.jP[k] == oc.last ? kNoStop : oc.jP[k];
         r.jV[k] = oc.jV[k];
       }
       r.ntri = 0;
