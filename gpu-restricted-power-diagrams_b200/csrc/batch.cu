@@ -750,7 +750,9 @@ int capture(rpd_batch *b) {
     if (G[d].T_ahead > 0) Tlater = std::max(Tlater, std::min(grow(G[d].T0, G[d].max_extra), kMaxT));
   }
   const size_t slot0 = defer_slot_bytes(Pb[0], Vb[0], Tslot0);
-  const size_t items0 = size_t(cap0) * std::max(1, (Tslot0 + chunk - 1) / chunk);
+  size_t surface = 0;
+  for (const rpd_solver *s : b->solvers) surface += size_t(s->grid_triangles);
+  const size_t items0 = size_t(defer_items(size_t(cap0), Tslot0, surface));
   if (any_grid && defer) {
     if ((e = b->defer_slots.ensure(slot0 * cap0)) != cudaSuccess ||
         (e = b->defer_part.ensure(sizeof(double) * 4 * items0)) != cudaSuccess ||
@@ -897,9 +899,8 @@ int capture(rpd_batch *b) {
       dq.slot_bytes = defer_slot_bytes(Pb[j], Vb[j], Ts);
       dq.chunk = chunk;
       dq.inline_max = 16;
-      dq.max_chunks = std::max(1, (Ts + chunk - 1) / chunk);
-      const size_t by_slots = (slot0 * cap0) / dq.slot_bytes, by_items = items0 / dq.max_chunks;
-      dq.capacity = int(std::min<size_t>({size_t(cap0), by_slots, by_items}));
+      dq.items = int(items0);
+      dq.capacity = int(std::min<size_t>(size_t(cap0), (slot0 * cap0) / dq.slot_bytes));
       dq.slots = b->defer_slots.as<unsigned char>();
       dq.part = b->defer_part.as<double>();
       dq.fail = b->defer_fail.as<int>();

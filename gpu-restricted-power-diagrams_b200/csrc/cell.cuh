@@ -62,14 +62,15 @@ struct DeferQueue {
   // [0] cells parked, [1] next work item (cells with an inner apex), [2]
   // chunks taken, [3] the largest triangle count parked ahead
   // (CellLaunch::T_ahead), [4] next work item (cells with the reference's
-  // start corner); zeroed before a pass
+  // start corner), [5] cells that found a slot but no work items left, to be
+  // solved again (kParkOverflow); zeroed before a pass
   int *counters = nullptr;
   // Work items are chunks, numbered compactly: a parked cell takes its
   // chunks' range from counters[2] and writes its slot for each of them
-  int *chunk_slot = nullptr;       // capacity * max_chunks
-  double *part = nullptr;          // capacity * max_chunks * 4 partial moments, by work item
-  int *fail = nullptr;             // capacity * max_chunks: (triangle << 4) | status, or INT_MAX
-  int max_chunks = 0;              // ceil(T / chunk)
+  int items = 0;                   // work items the arrays below hold (defer_items)
+  int *chunk_slot = nullptr;       // items
+  double *part = nullptr;          // items * 4 partial moments
+  int *fail = nullptr;             // items: (triangle << 4) | status, or INT_MAX
   int chunk = kConeChunk;          // triangles per work item
   int inline_max = 16;             // cells with at most this many triangles stay inline
 };
@@ -202,7 +203,7 @@ struct CellLaunch {
 };
 constexpr int kParkOverflow = 101;  // internal status: the queue was full
 constexpr int kProbeMiss = 102;     // internal status: the outside probe proved nothing
-constexpr int kDeferCounters = 5;   // ints of DeferQueue::counters
+constexpr int kDeferCounters = 6;   // ints of DeferQueue::counters
 constexpr int kTraceRecord = 12;
 
 // Largest caps of one build: P <= 255 (uchar plane ids in the reference,
@@ -224,6 +225,21 @@ __host__ __device__ inline int t_ahead_cap(int P, int K, int T, int max_extra) {
     ahead = T;
   }
   return ahead;
+}
+
+// Work items for `capacity` parked cells of up to T triangles: what all of
+// them could need, but at most the larger of one item per 32 triangles and of
+// one per cell and surface triangle.  A triangle lies in a few cells, so with
+// an apex inside, whose cells keep the triangles they meet, the last holds
+// them all; cells that find none run again with their cones in their own
+// warp.  40 bytes each: worst-case arrays of items of 8 triangles took 3.2 GB
+// for 10M seeds at T 100 and 25.6 GB at T 1000, these 0.8 and 6.4.
+inline int defer_items(size_t capacity, int T, size_t surface) {
+  auto of = [&](int chunk) { return capacity * size_t(T > chunk ? (T + chunk - 1) / chunk : 1); };
+  const size_t most = of(kConeChunk), usual = of(32), near = capacity + surface;
+  const size_t items = usual > near ? usual : near;
+  const size_t limit = 0x7fffffff;
+  return int(most < items ? (most < limit ? most : limit) : (items < limit ? items : limit));
 }
 
 // Shared memory bytes one warp needs for these caps.

@@ -2042,8 +2042,26 @@ __device__ __forceinline__ int *slot_list(const DeferQueue &dq, int slot, const 
   return reinterpret_cast<int *>(base + sizeof(DeferHeader) + 32u * L.Pc + 44u * L.Vc);
 }
 
+// A slot taken for a cell whose restriction ended early: its status, no work
+// items (k_cone_finish writes every taken slot's cell).
+__device__ void park_fixed(const DeferQueue &dq, int slot, int diag, int sid, int status, int lane) {
+  if (lane == 0) {
+    DeferHeader *h = reinterpret_cast<DeferHeader *>(dq.slots + size_t(slot) * dq.slot_bytes);
+    h->sid = sid;
+    h->nuniq = 0;
+    h->nv = h->np = 0;
+    h->inner = 0;
+    h->diag = diag;
+    h->chunk_base = 0;
+    h->fixed = status;
+    for (int d = 0; d < 4; ++d) h->acc[d] = 0.0;
+  }
+}
+
+// False when no work items are left: nothing is parked, and the slot names
+// itself in those that were (without triangles, so they are passed over).
 // list_in_place: the ids were gathered into the slot already.
-__device__ void park_cell(const WarpCell &w, const DeferQueue &dq, int slot, const Layout &L, int diag, int sid,
+__device__ bool park_cell(const WarpCell &w, const DeferQueue &dq, int slot, const Layout &L, int diag, int sid,
                           int nuniq, bool inner, const double acc[4], int lane, bool list_in_place = false) {
   const int T = L.T;
   unsigned char *base = dq.slots + size_t(slot) * dq.slot_bytes;
@@ -2054,9 +2072,12 @@ __device__ void park_cell(const WarpCell &w, const DeferQueue &dq, int slot, con
   unsigned *vt = reinterpret_cast<unsigned *>(vd + L.Vc);
   int *tl = reinterpret_cast<int *>(vt + L.Vc);
   const int nch = (nuniq + dq.chunk - 1) / dq.chunk;
-  int cb = 0;
+  int cb = lane == 0 ? atomicAdd(&dq.counters[2], nch) : 0;
+  cb = __shfl_sync(kFull, cb, 0);
+  const int room = max(0, dq.items - cb);
+  for (int c = lane; c < min(nch, room); c += 32) dq.chunk_slot[cb + c] = slot;
+  if (nch > room) return false;
   if (lane == 0) {
-    cb = atomicAdd(&dq.counters[2], nch);
     h->sid = sid;
     h->nuniq = nuniq;
     h->nv = w.nv;
@@ -2068,8 +2089,6 @@ __device__ void park_cell(const WarpCell &w, const DeferQueue &dq, int slot, con
     for (int d = 0; d < 3; ++d) h->pt0[d] = w.pts[d];
     for (int d = 0; d < 4; ++d) h->acc[d] = acc[d];
   }
-  cb = __shfl_sync(kFull, cb, 0);
-  for (int c = lane; c < nch; c += 32) dq.chunk_slot[cb + c] = slot;
   for (int i = lane; i < w.np; i += 32) pl[i] = w.plane[i];
   if (inner) {
     // the cone kernel needs the vertices' positions and the faces: built once
@@ -2104,22 +2123,7 @@ __device__ void park_cell(const WarpCell &w, const DeferQueue &dq, int slot, con
     int *nb = tl + ((T + 3) & ~3);
     for (int i = lane; i < w.np; i += 32) nb[i] = w.pnb[i];
   }
-}
-
-// A slot taken for a cell parked ahead whose restriction ended early: its
-// status, no work items (k_cone_finish writes every taken slot's cell).
-__device__ void park_fixed(const DeferQueue &dq, int slot, int diag, int sid, int status, int lane) {
-  if (lane == 0) {
-    DeferHeader *h = reinterpret_cast<DeferHeader *>(dq.slots + size_t(slot) * dq.slot_bytes);
-    h->sid = sid;
-    h->nuniq = 0;
-    h->nv = h->np = 0;
-    h->inner = 0;
-    h->diag = diag;
-    h->chunk_base = 0;
-    h->fixed = status;
-    for (int d = 0; d < 4; ++d) h->acc[d] = 0.0;
-  }
+  return true;
 }
 
 // The record of a cell of a retry pass (CellLaunch::retry), whose caps no
@@ -2346,7 +2350,12 @@ __device__ int restrict_to_domain(WarpCell &w, const CellLaunch &a, const Layout
   }
   if (slot < dq.capacity) {
     // park the cell: its triangles become work items of k_cone
-    park_cell(w, dq, slot, L, a.diag, sid_of_cell, nuniq, inner, acc, lane, ahead);
+    if (!park_cell(w, dq, slot, L, a.diag, sid_of_cell, nuniq, inner, acc, lane, ahead)) {
+      // no work items left: as where no slot is
+      park_fixed(dq, slot, a.diag, sid_of_cell, ahead ? kTriangleOverflow : kParkOverflow, lane);
+      if (!ahead && lane == 0) atomicAdd(&dq.counters[5], 1);
+      return kDeferred;
+    }
     // the retry passes' T schedule follows the counts settled ahead
     if (ahead && lane == 0 && !late && ntr <= a.T_sure) atomicMax(a.ahead_max ? a.ahead_max : &dq.counters[3], ntr);
     return kDeferred;
@@ -3036,8 +3045,9 @@ __global__ void __launch_bounds__(128, 6) k_probe_batch(const ProbeLaunch *__res
 // Rows of many diagrams in one persistent launch (batched solves): diagram
 // d owns rows start[d] .. start[d+1] and its own launch record descs[d];
 // warps stride over the rows.  park_counter, left (optional): the re-run of
-// the cells that found the defer queue full or that the octet clipping left
-// (ClipHand::ctr[2]), which exits when there are none.
+// the cells that found the defer queue full (park_counter: its counters) or
+// that the octet clipping left (ClipHand::ctr[2]), which exits when there are
+// none.
 // work (optional, zeroed before the launch): warps take their rows one at a
 // time from this counter (persistent launches of unknown row counts, so a
 // warp that drew heavy rows does not hold the launch back); null: warp w
@@ -3048,7 +3058,9 @@ __global__ void __launch_bounds__(128, 5)
                  const __grid_constant__ Layout L, int only_status, const int *__restrict__ park_counter,
                  int park_capacity, const int *__restrict__ left, int *__restrict__ work) {
   extern __shared__ __align__(16) unsigned char smem[];
-  if ((park_counter || left) && !(park_counter && *park_counter > park_capacity) && !(left && *left > 0)) return;
+  if ((park_counter || left) && !(park_counter && (park_counter[0] > park_capacity || park_counter[5] > 0)) &&
+      !(left && *left > 0))
+    return;
   const int lane = threadIdx.x & 31;
   unsigned char *wsmem = smem + size_t(threadIdx.x >> 5) * L.total;
   const int total = start[ndiag];
@@ -3099,7 +3111,7 @@ template <int VS, class Desc, int MODE = kConeAll>
 __device__ __forceinline__ void cone_items(const DeferQueue &dq, const Layout &L, Desc desc, unsigned char *wsmem,
                                            int lane) {
   WarpCell w = bind(wsmem, L);
-  const int items = min(*(volatile int *)&dq.counters[2], dq.capacity * dq.max_chunks);
+  const int items = min(*(volatile int *)&dq.counters[2], dq.items);
   int *next = &dq.counters[MODE == kConeCorner ? 4 : 1];
   for (;;) {
     int item = 0;

@@ -27,7 +27,7 @@ cudaError_t cell_launch_prec(const CellLaunch &a, cudaStream_t st, int sm_count,
   if (a.T_ahead > kMaxT || (a.T_ahead > a.T && (!a.defer.slots || a.hess))) return cudaErrorInvalidValue;
   const Layout L = make_layout(a.P, a.V, a.T, a.grid.size > 0, a.hess ? a.HC : 0, a.T_ahead, a.precision,
                                a.grid.lists_disjoint != 0);
-  if (a.defer.slots && (a.defer.slot_bytes < slot_bytes_for(L, L.T) || a.defer.max_chunks * a.defer.chunk < L.T))
+  if (a.defer.slots && (a.defer.slot_bytes < slot_bytes_for(L, L.T) || a.defer.items < 1))
     return cudaErrorInvalidValue;
   const int vs = L.Vc / 32;
   if (a.precision == 1) return launch_prec<1>(a, L, vs, st, sm_count, launches);

@@ -13,7 +13,7 @@ cudaError_t cell_launch_safe(const CellLaunch &a, cudaStream_t st, int sm_count,
   if (a.T_ahead > kMaxT || (a.T_ahead > a.T && (!a.defer.slots || a.hess))) return cudaErrorInvalidValue;
   const Layout L = make_layout(a.P, a.V, a.T, a.grid.size > 0, a.hess ? a.HC : 0, a.T_ahead, 0,
                                a.grid.lists_disjoint != 0);
-  if (a.defer.slots && (a.defer.slot_bytes < slot_bytes_for(L, L.T) || a.defer.max_chunks * a.defer.chunk < L.T))
+  if (a.defer.slots && (a.defer.slot_bytes < slot_bytes_for(L, L.T) || a.defer.items < 1))
     return cudaErrorInvalidValue;
   const int vs = L.Vc / 32;
   if (vs <= 2) return launch_vs<2, 0, 1>(a, L, st, sm_count, launches);
@@ -29,7 +29,7 @@ cudaError_t cell_batch_launch_safe(const CellBatch &b, cudaStream_t st, int sm_c
   if (b.HC && b.defer.slots) return cudaErrorInvalidValue;  // Hessian rows are summed inline
   const Layout Lg = make_layout(b.P, b.V, b.T, true, b.HC, b.T_slot, 0, b.disjoint),
                Lp = make_layout(b.P, b.V, b.T, false, b.HC);
-  if (b.defer.slots && (b.defer.slot_bytes < slot_bytes_for(Lg, Lg.T) || b.defer.max_chunks * b.defer.chunk < Lg.T))
+  if (b.defer.slots && (b.defer.slot_bytes < slot_bytes_for(Lg, Lg.T) || b.defer.items < 1))
     return cudaErrorInvalidValue;
   const int vs = Lg.Vc / 32;
   if (vs <= 2) return launch_batch_vs<2, 1>(b, Lg, Lp, st, sm_count, launches);

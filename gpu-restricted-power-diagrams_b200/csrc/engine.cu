@@ -743,10 +743,10 @@ int run_pass(rpd_solver *s, const int *ids, int num, int K, int P, int V, int T,
     dq.slot_bytes = defer_slot_bytes(P, V, t_slot);
     dq.chunk = kConeChunk;
     dq.inline_max = 16;
-    dq.max_chunks = std::max(1, (t_slot + dq.chunk - 1) / dq.chunk);
+    dq.items = defer_items(size_t(dq.capacity), t_slot, size_t(s->grid_triangles));
     a.T_ahead = T_ahead > T ? T_ahead : 0;
     a.out_domain_ahead = out_domain_ahead;
-    const size_t items = size_t(dq.capacity) * dq.max_chunks;
+    const size_t items = size_t(dq.items);
     if ((e = s->defer_slots.ensure(dq.slot_bytes * dq.capacity)) != cudaSuccess) return map_cuda(ctx, e, "alloc defer");
     if ((e = s->defer_part.ensure(sizeof(double) * 4 * items)) != cudaSuccess) return map_cuda(ctx, e, "alloc defer");
     if ((e = s->defer_fail.ensure(sizeof(int) * items)) != cudaSuccess) return map_cuda(ctx, e, "alloc defer");
@@ -796,7 +796,7 @@ int run_pass(rpd_solver *s, const int *ids, int num, int K, int P, int V, int T,
     if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return map_cuda(ctx, e, "cell kernel");
     const int parked = ctrs[0];
     if (a.T_ahead > 0) s->ahead_max = std::max(s->ahead_max, ctrs[3]);
-    if (parked > a.defer.capacity || hctr[2] > 0) {
+    if (parked > a.defer.capacity || ctrs[5] > 0 || hctr[2] > 0) {
       CellLaunch b = a;
       b.hand = ClipHand();
       b.defer = DeferQueue();

@@ -36,6 +36,7 @@ double ms_between(Clock::time_point a, Clock::time_point b) {
 struct Session {
   int id = 0;
   int n = 0;                     // seeds
+  size_t surface = 0;            // triangles of its domain (an estimate for one built on the device)
   rpd_solver *solver = nullptr;
   bool ready = false;            // solved once
   bool failed = false;           // its first solve failed
@@ -88,12 +89,20 @@ size_t grid_bytes(const rpd_grid *g) {
          size_t(nl) * 4 + 4096;
 }
 
-// Device bytes of a domain built on the device at size^3 voxels: flags,
-// offsets, summed tables, and for the reservation a surface of 48 size^2
-// triangles (the session's actual bytes replace it after its solve).
+size_t grid_triangles(const rpd_grid *g) {
+  int size = 0, np = 0, nt = 0, nl = 0;
+  return g && rpd_grid_info(g, &size, &np, &nt, &nl) == RPD_OK ? size_t(nt) : 0;
+}
+
+// For the reservation a domain built on the device at size^3 voxels has a
+// surface of 48 size^2 triangles (the session's actual bytes replace it after
+// its solve).
+size_t device_grid_triangles(int size) { return 48 * size_t(size) * size_t(size); }
+
+// Its device bytes: flags, offsets, summed tables, the surface.
 size_t device_grid_bytes(int size) {
   const size_t S = size_t(size), S1 = S + 1;
-  return S * S * S * (1 + 4) + S1 * S1 * S1 * 8 + 48 * S * S * (12 + 4) + 24 * S * S * 16 + 4096;
+  return S * S * S * (1 + 4) + S1 * S1 * S1 * 8 + device_grid_triangles(size) * (12 + 4) + 24 * S * S * 16 + 4096;
 }
 
 // The build's workspace: per lattice point the field, edge mask, counts and
@@ -114,16 +123,18 @@ size_t resident_bytes(int n, const rpd_params &p) {
 // staging, parked boundary cells, neighbour rows of retry passes (caps grown
 // x1.5 up to 5 times: bounded by 8x the first caps, which also bounds the
 // first pass's slots for triangle overflows parked ahead).  Per work item of
-// the parked cells: partial moments, failure, owning slot (40 bytes).  Records
-// of the cells handed to a warp, and of those clipped past the caps (16 bytes).
-size_t transient_bytes(int n, const rpd_params &p) {
+// the parked cells: partial moments, failure, owning slot (40 bytes); surface:
+// the domain's triangles.  Records of the cells handed to a warp, and of
+// those clipped past the caps (16 bytes).
+size_t transient_bytes(int n, const rpd_params &p, size_t surface) {
   const size_t cap = std::min<size_t>(size_t(n), std::max<size_t>(32768, size_t(n) / 8));
   const size_t P = size_t(std::min(255, p.P * 8)), V = size_t(std::min(256, p.V * 8)),
                T = size_t(std::min(4096, p.T * 8));
   const size_t slot = 144 + 32 * P + 44 * V + 4 * T;
   // --hessian: the rows on the device and their user-order staging
   const size_t hess = p.hessian_h > 0 ? 2 * size_t(n) * size_t(p.hessian_h) * (8 * size_t(p.hessian_hc) + 4) : 0;
-  return size_t(n) * (12 + 16 + 32 + 12 + 16) + cap * (slot / 4 + 40 * (T / rpd::kConeChunk + 1) / 4) +
+  return size_t(n) * (12 + 16 + 32 + 12 + 16) + cap * (slot / 4) +
+         40 * (size_t(rpd::defer_items(cap, int(T), 0)) / 4 + surface) +
          size_t(rpd::clip_hand_capacity(n)) * rpd::kClipRecordBytes +
          size_t(n) / 4 * size_t(p.K) * 8 * 4 + hess + (size_t(1) << 20);
 }
@@ -393,7 +404,8 @@ int submit_new(rpd_server *sv, std::unique_ptr<Request> r, const float *xyzw, in
     r->hessian = hessian;
     r->hessian_ids = hessian_ids;
   }
-  r->need = transient_bytes(n, r->params);
+  const size_t surface = r->grid ? grid_triangles(r->grid) : device_grid_triangles(r->dom_size);
+  r->need = transient_bytes(n, r->params, surface);
   r->new_resident = resident_bytes(n, r->params);
   if (r->dom_kind != kDomHost) {
     r->need += device_grid_build_bytes(r->dom_size);
@@ -408,6 +420,7 @@ int submit_new(rpd_server *sv, std::unique_ptr<Request> r, const float *xyzw, in
   auto s = std::make_unique<Session>();
   s->id = sv->next_session++;
   s->n = n;
+  s->surface = surface;
   s->pending = 1;
   r->session = s->id;
   if (session) *session = s->id;
@@ -480,7 +493,7 @@ int rpd_server_submit_reweight_hessian(rpd_server *sv, int session, const float 
   Session *s = it->second.get();
   r->n = s->n;
   r->data.assign(w, w + size_t(s->n));
-  r->need = transient_bytes(s->n, r->params);
+  r->need = transient_bytes(s->n, r->params, s->surface);
   s->pending += 1;
   return sv->submit(std::move(r));
 }
