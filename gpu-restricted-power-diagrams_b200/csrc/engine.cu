@@ -23,11 +23,11 @@ cudaStream_t g_alloc_stream[kMaxDev] = {};
 struct Kept {
   std::mutex mu;
   std::map<size_t, std::vector<void *>> blocks;
-  size_t bytes = 0;
+  size_t bytes = 0, most = 0;  // most: set by the first context
   int contexts = 0;
 };
 Kept *const g_kept = new Kept[kMaxDev];
-constexpr size_t kKeepBlock = size_t(1) << 30, kKeepBytes = size_t(8) << 30;
+constexpr size_t kKeepBlock = size_t(1) << 30;
 
 size_t size_class(size_t bytes) {
   size_t step = 512;
@@ -53,16 +53,26 @@ cudaError_t alloc_stream(int dev, cudaStream_t *out) {
 }
 }  // namespace pool_detail
 
-// Returns the kept blocks of a device to the driver's pool.
-static void pool_flush(int dev) {
+void pool_trim(int dev, size_t most) {
   using namespace pool_detail;
+  if (dev < 0 || dev >= kMaxDev) return;
+  Kept &k = g_kept[dev];
+  std::lock_guard<std::mutex> lock(k.mu);
   cudaStream_t st;
-  if (alloc_stream(dev, &st) != cudaSuccess) return;
-  std::lock_guard<std::mutex> lock(g_kept[dev].mu);
-  for (auto &c : g_kept[dev].blocks)
-    for (void *p : c.second) cudaFreeAsync(p, st);
-  g_kept[dev].blocks.clear();
-  g_kept[dev].bytes = 0;
+  if (k.bytes <= most || alloc_stream(dev, &st) != cudaSuccess) return;
+  while (k.bytes > most && !k.blocks.empty()) {
+    const auto c = std::prev(k.blocks.end());  // the largest first
+    if (!c->second.empty()) {
+      cudaFreeAsync(c->second.back(), st);
+      c->second.pop_back();
+      k.bytes -= c->first;
+    }
+    if (c->second.empty()) k.blocks.erase(c);
+  }
+}
+
+size_t pool_block(size_t bytes) {
+  return bytes > 0 && bytes <= pool_detail::kKeepBlock ? pool_detail::size_class(bytes) : bytes;
 }
 
 cudaError_t pool_alloc(void **p, size_t bytes, int *device) {
@@ -73,7 +83,7 @@ cudaError_t pool_alloc(void **p, size_t bytes, int *device) {
   if (e != cudaSuccess || (e = alloc_stream(dev, &st)) != cudaSuccess) return e;
   *device = dev;
   if (bytes <= kKeepBlock) {
-    bytes = size_class(bytes);
+    bytes = pool_block(bytes);
     std::lock_guard<std::mutex> lock(g_kept[dev].mu);
     auto c = g_kept[dev].blocks.find(bytes);
     if (c != g_kept[dev].blocks.end() && !c->second.empty()) {
@@ -85,7 +95,7 @@ cudaError_t pool_alloc(void **p, size_t bytes, int *device) {
   }
   if ((e = cudaMallocAsync(p, bytes, st)) == cudaErrorMemoryAllocation) {
     cudaGetLastError();
-    pool_flush(dev);
+    pool_trim(dev, 0);
     e = cudaMallocAsync(p, bytes, st);
   }
   if (e != cudaSuccess) return e;
@@ -96,9 +106,9 @@ cudaError_t pool_alloc(void **p, size_t bytes, int *device) {
 void pool_free(void *p, size_t bytes, int dev) {
   using namespace pool_detail;
   if (bytes <= kKeepBlock) {
-    bytes = size_class(bytes);
+    bytes = pool_block(bytes);
     std::lock_guard<std::mutex> lock(g_kept[dev].mu);
-    if (g_kept[dev].contexts > 0 && g_kept[dev].bytes + bytes <= kKeepBytes) {
+    if (g_kept[dev].contexts > 0 && g_kept[dev].bytes + bytes <= g_kept[dev].most) {
       try {
         g_kept[dev].blocks[bytes].push_back(p);
         g_kept[dev].bytes += bytes;
@@ -111,16 +121,17 @@ void pool_free(void *p, size_t bytes, int dev) {
   if (alloc_stream(dev, &st) == cudaSuccess) cudaFreeAsync(p, st);
 }
 
-void pool_context(int dev, int change) {
+void pool_context(int dev, int change, size_t device_bytes) {
   using namespace pool_detail;
   if (dev < 0 || dev >= kMaxDev) return;
   bool last;
   {
     std::lock_guard<std::mutex> lock(g_kept[dev].mu);
     g_kept[dev].contexts += change;
+    if (device_bytes) g_kept[dev].most = device_bytes / 32;
     last = g_kept[dev].contexts <= 0;
   }
-  if (last) pool_flush(dev);
+  if (last) pool_trim(dev, 0);
 }
 
 namespace {
@@ -858,7 +869,7 @@ rpd_context *rpd_context_create(int device, int *err) {
     if (err) *err = RPD_ERR_CUDA;
     return nullptr;
   }
-  pool_context(device, 1);
+  pool_context(device, 1, prop.totalGlobalMem);
   if (err) *err = RPD_OK;
   return ctx;
 }
@@ -1789,7 +1800,7 @@ size_t solver_device_bytes(const rpd_solver *s) {
                        &s->ids_c, &s->fail_ws, &s->hist, &s->gather, &s->defer_slots, &s->defer_part, &s->defer_fail,
                        &s->defer_ctr, &s->defer_chunk_slot, &s->hand_recs, &s->hand_ctr, &s->ahead, &s->wmin, &s->used, &s->hess, &s->hessid};
   size_t t = 0;
-  for (const DevBuf *x : b) t += x->bytes;
+  for (const DevBuf *x : b) t += pool_block(x->bytes);
   return t;
 }
 

@@ -22,15 +22,19 @@ namespace rpd {
 //
 // Freed blocks of up to 1 GB are kept by size class (eight steps per power of
 // two, so up to 1/8 of a block is unused) and handed out again without a call
-// into the driver, up to 8 GB per device while a context of the device
-// exists.  The driver's pool alone puts a large block together from
+// into the driver, up to 1/32 of the device's memory while a context of the
+// device exists; the serving loop gives back what its budget does not hold
+// (pool_trim).  The driver's pool alone puts a large block together from
 // fragments where freed blocks of other sizes lie in between; that took 10 to
 // 160 ms each (192 MB of parked cells' slots) and stopped all streams: twelve
 // requests on four streams took 0.1 to 1.5 s instead of 50 ms in one burst of
 // eight.
 cudaError_t pool_alloc(void **p, size_t bytes, int *device);
 void pool_free(void *p, size_t bytes, int device);
-void pool_context(int device, int change);  // a context made (1) or destroyed (-1)
+void pool_context(int device, int change, size_t device_bytes = 0);  // a context made (1) or destroyed (-1)
+// Gives kept blocks back to the driver's pool until at most `most` bytes are kept.
+void pool_trim(int device, size_t most);
+size_t pool_block(size_t bytes);  // the block's size for an allocation of `bytes`
 
 struct DevBuf {
   void *ptr = nullptr;

@@ -112,6 +112,9 @@ size_t device_grid_build_bytes(int size) {
   return S1 * S1 * S1 * (4 + 1 + 4 + 4) + (S * S * S + 1) * 4 + (size_t(1) << 20);
 }
 
+// Buffers take whole blocks, up to 1/8 larger (pool_block).
+size_t in_blocks(size_t bytes) { return bytes + bytes / 8; }
+
 // Device bytes a session keeps: seeds (given and binned), permutation and
 // inverse, neighbour table, results, status, bins.
 size_t resident_bytes(int n, const rpd_params &p) {
@@ -176,6 +179,9 @@ struct rpd_server {
         continue;
       }
       queue.erase(it);
+      // the blocks that freed buffers left for reuse count too
+      const size_t used = resident + inflight + want;
+      rpd::pool_trim(device, used < budget ? budget - used : 0);
       return r;
     }
     return nullptr;
@@ -405,17 +411,17 @@ int submit_new(rpd_server *sv, std::unique_ptr<Request> r, const float *xyzw, in
     r->hessian_ids = hessian_ids;
   }
   const size_t surface = r->grid ? grid_triangles(r->grid) : device_grid_triangles(r->dom_size);
-  r->need = transient_bytes(n, r->params, surface);
-  r->new_resident = resident_bytes(n, r->params);
+  r->need = in_blocks(transient_bytes(n, r->params, surface));
+  r->new_resident = in_blocks(resident_bytes(n, r->params));
   if (r->dom_kind != kDomHost) {
-    r->need += device_grid_build_bytes(r->dom_size);
-    r->new_resident += device_grid_bytes(r->dom_size);
+    r->need += in_blocks(device_grid_build_bytes(r->dom_size));
+    r->new_resident += in_blocks(device_grid_bytes(r->dom_size));
   }
   std::lock_guard<std::mutex> lock(sv->mu);
   if (sv->stop) return RPD_ERR_INVALID;
   if (r->grid && !sv->grids.count(r->grid)) {
     sv->grids[r->grid] = std::make_unique<GridHolder>();
-    r->new_resident += grid_bytes(r->grid);  // reserved with the first session on it
+    r->new_resident += in_blocks(grid_bytes(r->grid));  // reserved with the first session on it
   }
   auto s = std::make_unique<Session>();
   s->id = sv->next_session++;
@@ -493,7 +499,7 @@ int rpd_server_submit_reweight_hessian(rpd_server *sv, int session, const float 
   Session *s = it->second.get();
   r->n = s->n;
   r->data.assign(w, w + size_t(s->n));
-  r->need = transient_bytes(s->n, r->params, s->surface);
+  r->need = in_blocks(transient_bytes(s->n, r->params, s->surface));
   s->pending += 1;
   return sv->submit(std::move(r));
 }

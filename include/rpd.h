@@ -397,7 +397,8 @@ int rpd_solver_get_used(rpd_solver *s, double *rows4, int *user_ids, rpd_mem whe
  * Requests -- a new session's solve, or a weight-only re-solve of a session --
  * are admitted in arrival order as one of `slots` concurrent streams and
  * device memory free up: resident sessions plus the requests in flight stay
- * within mem_budget bytes (0: 90% of the free memory).  A session runs one
+ * within mem_budget bytes (0: 90% of the free memory); freed memory that the
+ * library keeps for reuse is given back where it would not fit beside them.  A session runs one
  * request at a time; requests of different sessions overlap on the device.
  * A request's result depends only on its own inputs. */
 typedef struct rpd_server rpd_server;
