@@ -764,7 +764,10 @@ int capture(rpd_batch *b) {
   if ((e = b->work.ensure(sizeof(int))) != cudaSuccess) return map_cuda(ctx, e, "alloc batch");
   ClipHand hand;
   if (!any_safe) {
-    hand.capacity = clip_hand_capacity(int(cells));
+    // with Hessian rows nearly every cell of the diagram is handed over
+    long long all = 0;
+    for (int d = 0; d < nd; ++d) all += G[d].H > 0 ? G[d].n : 0;
+    hand.capacity = int(std::min(cells, clip_hand_capacity(int(cells)) + all));
     if ((e = b->hand_recs.ensure(size_t(kClipRecordBytes) * hand.capacity)) != cudaSuccess ||
         (e = b->hand_ctr.ensure(sizeof(int) * kClipCounters)) != cudaSuccess)
       return map_cuda(ctx, e, "alloc batch clip records");

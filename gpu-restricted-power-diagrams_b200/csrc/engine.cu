@@ -787,8 +787,15 @@ int run_pass(rpd_solver *s, const int *ids, int num, int K, int P, int V, int T,
     ClipHand &hd = a.hand;
     // a retry pass whose recorded cells are settled holds boundary cells only,
     // every one handed over: it may use all of the first pass's records (5M
-    // blue-noise seeds' second pass 26.0 -> 9 ms)
+    // blue-noise seeds' second pass 26.0 -> 9 ms).  With Hessian rows or used
+    // cells nearly every cell is handed over, and one without a record is
+    // clipped twice: 400K lattice seeds in a cube, used cells 19.4 -> 8.2
+    // ms, rows 32.7 -> 18.2
     hd.capacity = std::max(clip_hand_capacity(num), std::min(num, clip_hand_capacity(s->n)));
+    if (a.hess || a.used) {
+      if (s->hand_recs.ensure(size_t(kClipRecordBytes) * num) == cudaSuccess) hd.capacity = num;
+      else cudaGetLastError();  // the smaller array will do
+    }
     if ((e = s->hand_recs.ensure(size_t(kClipRecordBytes) * hd.capacity)) != cudaSuccess ||
         (e = s->hand_ctr.ensure(sizeof(int) * kClipCounters)) != cudaSuccess)
       return map_cuda(ctx, e, "alloc clip records");

@@ -149,7 +149,8 @@ void solver_share_grid(rpd_solver *dst, const rpd_solver *src);
 size_t solver_device_bytes(const rpd_solver *s);
 void solver_trim(rpd_solver *s);
 // Records for the clipped cells of a launch that need a warp: its boundary
-// cells, whose share falls as the cell count grows.
+// cells, whose share falls as the cell count grows.  (Launches with Hessian
+// rows or used cells hand over all of their cells.)
 int clip_hand_capacity(int num);
 
 }  // namespace rpd

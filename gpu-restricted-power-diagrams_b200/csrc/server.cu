@@ -138,7 +138,7 @@ size_t transient_bytes(int n, const rpd_params &p, size_t surface) {
   const size_t hess = p.hessian_h > 0 ? 2 * size_t(n) * size_t(p.hessian_h) * (8 * size_t(p.hessian_hc) + 4) : 0;
   return size_t(n) * (12 + 16 + 32 + 12 + 16) + cap * (slot / 4) +
          40 * (size_t(rpd::defer_items(cap, int(T), 0)) / 4 + surface) +
-         size_t(rpd::clip_hand_capacity(n)) * rpd::kClipRecordBytes +
+         size_t(p.hessian_h > 0 || p.keep_distance >= 0 ? n : rpd::clip_hand_capacity(n)) * rpd::kClipRecordBytes +
          size_t(n) / 4 * size_t(p.K) * 8 * 4 + hess + (size_t(1) << 20);
 }
 
