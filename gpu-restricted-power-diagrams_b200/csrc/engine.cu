@@ -617,45 +617,51 @@ int run_probe(rpd_solver *s, int P, int V, float eps, int *ids, int &nmiss, int 
   return RPD_OK;
 }
 
-// The neighbour-search variant for K rows of this solver (rpd::KnnVariant).
-// RPD_FLAG_KNN_WARP / RPD_FLAG_KNN_THREAD force one.  Otherwise the
-// context's choice for K.  Above kKnnTrialMaxK a warp per seed: it was the
+// The neighbour-search variant for `num` rows of K (rpd::KnnVariant).
+// RPD_FLAG_KNN_WARP / RPD_FLAG_KNN_THREAD force one, a pin of the context's
+// comes next.  Otherwise, above kKnnTrialMaxK a warp per seed: it was the
 // faster of the two on every input measured (K 50: 1.90 against 3.04 ms for 1M
 // lattice seeds, 1.00 / 1.82 for 500K uniform ones, 0.23 / 0.58 for 100K).
-// Up to it, a trial the first time K comes up with enough rows to tell: both
-// variants run on the first quarter of the rows (a thread per seed needs
-// some 100K rows to fill the GPU: K 20, 0.18 / 0.21 ms for 100K seeds but 3.1
-// / 2.1 ms for 2M), one untimed round, one timed with events, into `out`,
-// which the real launch then overwrites; both give the same lists, so only
-// their speed differs.  Fewer rows than a trial takes (retry passes): a warp
-// per seed -- a thread per seed leaves most of the GPU idle there and each
-// row's search serial (0.45 ms for 144 rows).
-constexpr int kKnnTrialMaxK = 32;
-
-int knn_variant_for(rpd_solver *s, const int *ids, int num, int K, unsigned *out, unsigned flags) {
+// Up to it the context's choice for K and the power of two below num, made by
+// a trial the first time that the two come up: a thread per seed needs some
+// 100K rows to fill the GPU, so the winner depends on the row count (uniform
+// seeds, warp / thread: K 8, 0.08 / 0.13 ms for 32K and 0.45 / 0.21 for 192K;
+// K 20, 0.06 / 0.17 and 0.32 / 0.32, 3.4 / 2.4 for 2M).  The trial runs both on
+// all rows, timed with events, after an untimed one on few; both write the
+// same lists into `out`, so *done: the search itself is not run again.  Fewer
+// rows than a trial takes (retry passes): a warp per seed -- a thread per
+// seed leaves most of the GPU idle there and each row's search serial (0.45
+// ms for 144 rows).
+int knn_variant_for(rpd_solver *s, const int *ids, int num, int K, unsigned *out, unsigned flags, bool *done) {
+  *done = false;
   if (flags & RPD_FLAG_KNN_WARP) return kKnnWarp;
   if (flags & RPD_FLAG_KNN_THREAD) return K <= kKnnThreadMaxK ? kKnnThread : kKnnWarp;
-  constexpr int kTrialRows = 16384;
+  constexpr int kTrialRows = 16384, kWarmRows = 2048;
   if (K > kKnnThreadMaxK || num < kTrialRows) return kKnnWarp;
   rpd_context *ctx = s->ctx;
-  if (ctx->knn_variant[K] >= 0) return ctx->knn_variant[K];
-  if (K > kKnnTrialMaxK) return ctx->knn_variant[K] = kKnnWarp;
-  const int m = std::max(kTrialRows, std::min(num / 4, 262144));
-  cudaStream_t st = ctx->stream;
-  Events<4> ev;
-  float ms[2] = {0.f, 0.f};
-  for (int round = 0; round < 2; ++round)
-    for (int v = 0; v < 2; ++v) {
-      if (round) cudaEventRecord(ev[2 * v], st);
-      if (knn_launch(s->stored.as<float4>(), s->counters.as<int>(), s->dim, ids, m, K, s->ring_bound.as<float>(),
-                     out, nullptr, st, v) != cudaSuccess)
-        return kKnnWarp;
-      if (round) cudaEventRecord(ev[2 * v + 1], st);
-    }
-  if (cudaEventSynchronize(ev[3]) != cudaSuccess) return kKnnWarp;
-  for (int v = 0; v < 2; ++v) cudaEventElapsedTime(&ms[v], ev[2 * v], ev[2 * v + 1]);
-  ctx->knn_variant[K] = ms[kKnnThread] < ms[kKnnWarp] ? kKnnThread : kKnnWarp;
-  return ctx->knn_variant[K];
+  if (ctx->knn_pin[K] >= 0) return ctx->knn_pin[K];
+  if (K > kKnnTrialMaxK) return ctx->knn_last[K] = kKnnWarp;
+  int size = 0;
+  while ((num >> size) > 1) ++size;
+  signed char &choice = ctx->knn_choice[K][size];
+  if (choice < 0) {
+    cudaStream_t st = ctx->stream;
+    Events<4> ev;
+    float ms[2] = {0.f, 0.f};
+    for (int round = 0; round < 2; ++round)
+      for (int v = 0; v < 2; ++v) {
+        if (round) cudaEventRecord(ev[2 * v], st);
+        if (knn_launch(s->stored.as<float4>(), s->counters.as<int>(), s->dim, ids, round ? num : kWarmRows, K,
+                       s->ring_bound.as<float>(), out, nullptr, st, v) != cudaSuccess)
+          return kKnnWarp;
+        if (round) cudaEventRecord(ev[2 * v + 1], st);
+      }
+    if (cudaEventSynchronize(ev[3]) != cudaSuccess) return kKnnWarp;
+    for (int v = 0; v < 2; ++v) cudaEventElapsedTime(&ms[v], ev[2 * v], ev[2 * v + 1]);
+    choice = ms[kKnnThread] < ms[kKnnWarp] ? kKnnThread : kKnnWarp;
+    *done = true;
+  }
+  return ctx->knn_last[K] = choice;
 }
 
 // Launches of fewer rows clip with a warp per cell: an octet's cell takes
@@ -690,10 +696,13 @@ int run_pass(rpd_solver *s, const int *ids, int num, int K, int P, int V, int T,
   cudaEventRecord(ev[0], st);
   if (!reuse) {
     if (all_cells) s->knn_full_K = 0;
-    const int variant = knn_variant_for(s, ids, num, Kx, kb.as<unsigned>(), s->launch_flags);
+    bool done = false;
+    const int variant = knn_variant_for(s, ids, num, Kx, kb.as<unsigned>(), s->launch_flags, &done);
     if (pi < 8) S.pass_knn_variant[pi] = variant;
-    e = knn_launch(s->stored.as<float4>(), s->counters.as<int>(), s->dim, ids, num, Kx, s->ring_bound.as<float>(),
-                   kb.as<unsigned>(), ctr ? ctr + RPD_CTR_NUM : nullptr, st, variant);
+    e = cudaSuccess;
+    if (!done || ctr)
+      e = knn_launch(s->stored.as<float4>(), s->counters.as<int>(), s->dim, ids, num, Kx, s->ring_bound.as<float>(),
+                     kb.as<unsigned>(), ctr ? ctr + RPD_CTR_NUM : nullptr, st, variant);
     if (e != cudaSuccess) return map_cuda(ctx, e, "knn");
     if (all_cells) {
       s->knn_full_K = K;
@@ -911,8 +920,12 @@ rpd_solver *rpd_solver_create(rpd_context *ctx, int *err) {
 int rpd_context_knn_variant(rpd_context *ctx, int K, int variant) {
   if (!ctx || K < 1 || K > kMaxK || variant < -2 || variant > 1) return RPD_ERR_INVALID;
   if (variant == kKnnThread && K > kKnnThreadMaxK) return RPD_ERR_CAPACITY;
-  if (variant != -2) ctx->knn_variant[K] = (signed char)variant;
-  return ctx->knn_variant[K];
+  if (variant != -2) {
+    ctx->knn_pin[K] = (signed char)variant;
+    ctx->knn_last[K] = -1;
+    if (K <= kKnnTrialMaxK) std::memset(ctx->knn_choice[K], -1, sizeof(ctx->knn_choice[K]));
+  }
+  return ctx->knn_pin[K] >= 0 ? ctx->knn_pin[K] : ctx->knn_last[K];
 }
 
 void rpd_solver_destroy(rpd_solver *s) {
@@ -1084,8 +1097,12 @@ int rpd_solver_knn(rpd_solver *s, int K, int *knn_user, rpd_mem where, float *de
   Events<2> ev;
   cudaEventRecord(ev[0], st);
   s->knn_full_K = 0;
-  e = knn_launch(s->stored.as<float4>(), s->counters.as<int>(), s->dim, nullptr, s->n, K, s->ring_bound.as<float>(),
-                 s->knn.as<unsigned>(), nullptr, st, knn_variant_for(s, nullptr, s->n, K, s->knn.as<unsigned>(), 0));
+  bool done = false;
+  const int variant = knn_variant_for(s, nullptr, s->n, K, s->knn.as<unsigned>(), 0, &done);
+  e = cudaSuccess;
+  if (!done)
+    e = knn_launch(s->stored.as<float4>(), s->counters.as<int>(), s->dim, nullptr, s->n, K, s->ring_bound.as<float>(),
+                   s->knn.as<unsigned>(), nullptr, st, variant);
   cudaEventRecord(ev[1], st);
   if (e != cudaSuccess) return map_cuda(ctx, e, "knn");
   s->knn_full_K = K;

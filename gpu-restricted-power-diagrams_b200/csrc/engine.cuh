@@ -75,10 +75,15 @@ struct rpd_context {
   int sm_count = 0;
   cudaStream_t stream = nullptr;
   std::string error;
-  // neighbour-search variant per K (rpd::KnnVariant), picked by a timed
-  // trial on this device the first time K comes up; -1 not tried yet
-  signed char knn_variant[257];
-  rpd_context() { std::memset(knn_variant, -1, sizeof(knn_variant)); }
+  // neighbour-search variants (rpd::KnnVariant, -1 none): pinned per K, the
+  // last one used for K, and per K and power of two of the rows the one picked
+  // by a timed trial on this device
+  signed char knn_pin[257], knn_last[257], knn_choice[rpd::kKnnTrialMaxK + 1][31];
+  rpd_context() {
+    std::memset(knn_pin, -1, sizeof(knn_pin));
+    std::memset(knn_last, -1, sizeof(knn_last));
+    std::memset(knn_choice, -1, sizeof(knn_choice));
+  }
 };
 
 struct rpd_solver {

@@ -24,6 +24,8 @@ void ring_bounds(int dim, float *bound);
 // are the same bit for bit.
 enum KnnVariant { kKnnWarp = 0, kKnnThread = 1 };
 constexpr int kKnnThreadMaxK = 128;
+// Up to this K searches of many rows choose their variant by a timed trial.
+constexpr int kKnnTrialMaxK = 32;
 cudaError_t knn_launch(const float4 *stored, const int *counters, int dim, const int *ids, int num, int K,
                        const float *ring_bound, unsigned *out, unsigned long long *candidates, cudaStream_t st,
                        int variant = kKnnWarp);

@@ -72,8 +72,9 @@ void *rpd_context_stream(rpd_context *ctx);
 const char *rpd_version(void);
 /* The neighbour-search variant the context uses for K (0: a warp per seed,
  * 1: a thread per seed, K <= 128): variant 0 or 1 pins it, -1 forgets it
- * (the next search with K times both again), -2 only reads it.  Returns the
- * variant for K afterwards, -1 when not chosen yet, or an rpd_error.  No
+ * (the next searches with K time both again), -2 only reads it.  Returns the
+ * variant of the last search with K (the choice depends on the number of rows
+ * too), -1 when none was chosen yet, or an rpd_error.  No
  * counterpart in the reference (one kernel, knearests.cl:36-78). */
 int rpd_context_knn_variant(rpd_context *ctx, int K, int variant);
 
@@ -229,8 +230,9 @@ rpd_grid *rpd_solver_export_grid(rpd_solver *s, int *err);
                                        shared-memory heap) for K <= 128 (same results).
                                        Without either flag, searches of at least 16K
                                        rows with K <= 32 use the variant each context
-                                       picks for K by a timed trial the first time K
-                                       comes up, others a warp per seed
+                                       picks by a timed trial the first time that K
+                                       and a row count of this power of two come up,
+                                       others a warp per seed
                                        (rpd_stats.pass_knn_variant) */
 
 /* VoroAlgo's knobs (voronoi.h:199-246; defaults of Options.cpp:22-28). */
