@@ -1,12 +1,12 @@
 // K-nearest neighbours on the binned seeds, one warp per seed (replaces the
 // reference's one-work-item heap search, knearests.cl:36-78).
 //
-// For K <= 96 (kSelectSlots) the warp first tries to select from the 5x5x5
-// bins around the seed's own (select_row): distances in registers, a
-// threshold that leaves between K and 32 S of them, one sort of those.  Where
-// that block does not decide (the K-th best lies past the third shell's
-// bound, more candidates than registers, ties across the threshold), and for
-// larger K, it scans shell by shell (merge_row):
+// For K of 7 (kSelectMinK) to 96 (kSelectSlots) the warp first tries to select
+// from the 5x5x5 bins around the seed's own (select_row): distances in
+// registers, a threshold that leaves between K and 32 S of them, one sort of
+// those.  Where that block does not decide (the K-th best lies past the
+// block's nearest face, more candidates than registers, ties across the
+// threshold), and for other K, it scans shell by shell (merge_row):
 //
 // Chebyshev shells of bins around the seed's bin.  Bins are
 // stored x-fastest, so every row of a shell is one contiguous range of the
@@ -96,7 +96,7 @@ struct ShellRows {
 // The K nearest of stored seed `pin` into row[0..K) (one warp), shell by
 // shell.
 template <int S>
-__device__ __noinline__ void merge_row(const float4 *__restrict__ stored, const int *__restrict__ counters, int dim,
+__device__ __forceinline__ void merge_row(const float4 *__restrict__ stored, const int *__restrict__ counters, int dim,
                                         int pin, int K, const float *__restrict__ ring_bound, unsigned *__restrict__ row,
                                         unsigned long long *__restrict__ candidates, unsigned long long *stage,
                                         int lane) {
@@ -208,13 +208,19 @@ __device__ __noinline__ void merge_row(const float4 *__restrict__ stored, const 
 // distances sit in registers (kSelectBatches per lane) and a threshold T with
 // K <= #(d <= T) <= 32 S is searched by counting (two or three counts: #
 // grows with T^1.5, so the next guess is interpolated); only the candidates
-// up to T are sorted.  The list is merge_row's bit for bit: the shells that
-// it scans are the block's -- it scans shell 2 since fewer than K candidates
-// lie below that shell's bound, and no further shell since K lie below shell
-// 3's -- and the K least keys are the same keys.  Measured: 1M lattice seeds
-// 3.26 -> 1.90 ms at K 50, 4.68 -> 2.75 at K 70, 2.42 -> 1.51 at K 20; 500K
-// uniform seeds 1.80 -> 1.00 ms at K 50.
+// up to T are sorted.  The list is merge_row's bit for bit: T lies where no
+// seed outside the shells that merge_row scans, or outside the block, can be,
+// so the K least keys are the same keys.  Measured against merge_row alone,
+// 300K uniform seeds: 1.01 -> 0.61 ms at K 50, 0.74 -> 0.48 at K 20, 2.07 ->
+// 1.39 at K 96; 1M lattice seeds at K 50 3.26 -> 1.90.  A row that is not
+// decided costs both: with the third shell's bound in place of the block's
+// face most rows of K 96 and those near the box's faces did (1.87 ms), and
+// with a fall-through where K lie below the second shell's bound those of K
+// <= 13 (K 8: 0.49 -> 0.69, now 0.44).  Up to K 6 the scan of 84 candidates
+// is the faster (K 1: 0.40 against 0.43 ms).  Seeds in dense clusters, whose
+// blocks hold more candidates than registers, pay 3 to 4%.
 constexpr int kSelectSlots = 3;    // K <= 96
+constexpr int kSelectMinK = 7;
 constexpr int kSelectBatches = 16; // 512 candidates (the block holds ~388)
 
 struct SelectSmem {
@@ -302,15 +308,35 @@ __device__ __forceinline__ bool select_row(const float4 *__restrict__ stored, co
     for (int b = 0; b < kSelectBatches; ++b) c += d[b] < t ? 1 : 0;
     return __reduce_add_sync(kFull, c);
   };
-  // merge_row's shells: shell 2 only if fewer than K lie below its bound, no
-  // shell past 2 if K lie below shell 3's or the block holds every bin
-  const float b2 = __ldg(&ring_bound[2]), b3 = __ldg(&ring_bound[3]);
-  if (below(__float_as_uint(b2)) >= K) return false;
-  int ch = below(__float_as_uint(b3));
-  if (ch < K) return false;
   // K <= #(d < t) <= 32 S
   constexpr int kMost = 32 * S;
-  unsigned t = __float_as_uint(b3);
+  // w / 1000 of the float roundings of a seed's bin, of a face's coordinate
+  // and of a distance are below this
+  constexpr float kFaceErr = 1e-3f;
+  const float w = 1000.f / float(dim);
+  unsigned t = __float_as_uint(__ldg(&ring_bound[2]));
+  int ch = below(t);
+  if (ch >= K) {
+    // merge_row stops before shell 2: its candidates all lie past the bound,
+    // but for the rounding
+    const float b = fmaxf(w - kFaceErr, 0.f);
+    if (below(__float_as_uint(b * b)) != ch) return false;
+  } else {
+    // merge_row scans shell 2, and further ones as long as fewer than K lie
+    // below their bounds; none of those holds a nearer candidate than the
+    // nearest face of the block with bins beyond
+    float face = 5.f * w;
+    if (cx > 2) face = fminf(face, p.x - float(cx - 2) * w);
+    if (cy > 2) face = fminf(face, p.y - float(cy - 2) * w);
+    if (cz > 2) face = fminf(face, p.z - float(cz - 2) * w);
+    if (cx + 3 < dim) face = fminf(face, float(cx + 3) * w - p.x);
+    if (cy + 3 < dim) face = fminf(face, float(cy + 3) * w - p.y);
+    if (cz + 3 < dim) face = fminf(face, float(cz + 3) * w - p.z);
+    face = fmaxf(face - kFaceErr, 0.f);
+    t = __float_as_uint(fmaxf(face * face, __ldg(&ring_bound[3])));
+    ch = below(t);
+    if (ch < K) return false;
+  }
   if (ch > kMost) {
     unsigned lo = 0, hi = t;
     const float want = 0.5f * float(K + kMost);
@@ -367,7 +393,7 @@ __device__ __forceinline__ void knn_row(const float4 *__restrict__ stored, const
                                         int pin, int K, const float *__restrict__ ring_bound, unsigned *__restrict__ row,
                                         unsigned long long *__restrict__ candidates, unsigned char *smem, int lane) {
   if constexpr (S <= kSelectSlots) {
-    if (select_row<S>(stored, counters, dim, pin, K, ring_bound, row, candidates,
+    if (K >= kSelectMinK && select_row<S>(stored, counters, dim, pin, K, ring_bound, row, candidates,
                       *reinterpret_cast<SelectSmem *>(smem), lane))
       return;
     __syncwarp();
