@@ -511,7 +511,9 @@ int describe(rpd_batch *b, std::vector<DiagStatic> &out) {
   cudaError_t e;
   out.assign(b->ndiag, DiagStatic{});
   bool any_safe = false;
+  long long cells = 0;
   for (const rpd_params &p : b->params) any_safe |= (p.flags & RPD_FLAG_SAFE_RADIUS) != 0;
+  for (const rpd_solver *s : b->solvers) cells += s->n;
   for (int d = 0; d < b->ndiag; ++d) {
     rpd_solver *s = b->solvers[d];
     const rpd_params &p = b->params[d];
@@ -532,8 +534,8 @@ int describe(rpd_batch *b, std::vector<DiagStatic> &out) {
     if ((e = s->ids_c.ensure(sizeof(int) * n)) != cudaSuccess) return map_cuda(ctx, e, "alloc ids");
     DiagStatic &g = out[d];
     // cells clipped past the first pass's caps, as rpd_solver_launch does
-    // (any size: the batch's cells share the launches)
-    const bool ahead = ahead_pays(p.K, p.V) && !any_safe && p.hessian_h == 0 && p.max_extra_passes > 0 &&
+    // (the batch's cells share the launches)
+    const bool ahead = ahead_pays(p.K, p.V) && cells >= kOctetMinRows && !any_safe && p.hessian_h == 0 && p.max_extra_passes > 0 &&
                        !(p.flags & RPD_FLAG_FIRST_PASS_ONLY);
     if (ahead && (e = s->ahead.ensure(sizeof(AheadRecord) * size_t(n))) != cudaSuccess)
       return map_cuda(ctx, e, "alloc records");
@@ -763,7 +765,7 @@ int capture(rpd_batch *b) {
   }
   if ((e = b->work.ensure(sizeof(int))) != cudaSuccess) return map_cuda(ctx, e, "alloc batch");
   ClipHand hand;
-  if (!any_safe) {
+  if (!any_safe && cells >= kOctetMinRows) {
     // with Hessian rows nearly every cell of the diagram is handed over
     long long all = 0;
     for (int d = 0; d < nd; ++d) all += G[d].H > 0 ? G[d].n : 0;

@@ -88,6 +88,16 @@ struct ClipHand {
   int *ctr = nullptr;
 };
 
+// Launches of fewer rows clip with a warp per cell: an octet's cell takes
+// longer than a warp's, which only more cells at a time repay (uniform seeds,
+// K 50, octet / warp: 2,000 rows 0.102 / 0.076 ms in the box and 0.145 /
+// 0.122 in a cube domain, 4,000 rows 0.109 / 0.127 and 0.156 / 0.189, 16,000
+// rows 0.205 / 0.377 and 0.295 / 0.547).  Batched launches whose rows only
+// the device knows hold both kernels, one of which returns at once (four
+// diagrams of 1K seeds in the box, every pass with eight lanes 1.23 ms, now
+// 0.96; eight of 2K 1.83 -> 1.54).
+constexpr int kOctetMinRows = 4096;
+
 // What a cell that failed a cap of the first pass needs, known since the
 // clipping went on past it (CellLaunch::ahead): the retry passes settle the
 // cell from this record instead of clipping it again.

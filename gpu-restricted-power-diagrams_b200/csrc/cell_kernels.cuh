@@ -36,7 +36,7 @@
 // vertex.  Integration (ConvexCell.cl:577-619) runs per vertex in double and
 // is reduced across the warp.
 #include <algorithm>
-
+#include <climits>
 #include <mutex>
 #include <set>
 #include <utility>
@@ -3048,6 +3048,7 @@ __global__ void __launch_bounds__(128, 6) k_probe_batch(const ProbeLaunch *__res
 // the cells that found the defer queue full (park_counter: its counters) or
 // that the octet clipping left (ClipHand::ctr[2]), which exits when there are
 // none.
+// below: launches of so many rows or more are another kernel's.
 // work (optional, zeroed before the launch): warps take their rows one at a
 // time from this counter (persistent launches of unknown row counts, so a
 // warp that drew heavy rows does not hold the launch back); null: warp w
@@ -3056,7 +3057,7 @@ template <int VS, bool GRID, bool INL, int SAFE = 0>
 __global__ void __launch_bounds__(128, 5)
     k_cell_batch(const CellLaunch *__restrict__ descs, const int *__restrict__ start, int ndiag,
                  const __grid_constant__ Layout L, int only_status, const int *__restrict__ park_counter,
-                 int park_capacity, const int *__restrict__ left, int *__restrict__ work) {
+                 int park_capacity, const int *__restrict__ left, int below, int *__restrict__ work) {
   extern __shared__ __align__(16) unsigned char smem[];
   if ((park_counter || left) && !(park_counter && (park_counter[0] > park_capacity || park_counter[5] > 0)) &&
       !(left && *left > 0))
@@ -3064,6 +3065,7 @@ __global__ void __launch_bounds__(128, 5)
   const int lane = threadIdx.x & 31;
   unsigned char *wsmem = smem + size_t(threadIdx.x >> 5) * L.total;
   const int total = start[ndiag];
+  if (total >= below) return;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
   int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (work) {
@@ -3347,11 +3349,11 @@ int resident_blocks(Kernel k, int threads, size_t smem, int sm_count) {
 
 // rows >= 0: the launch's row count is known: one warp per row.  Else a
 // persistent launch; with `work`, rows are taken from that counter (zeroed
-// here, on the stream).
+// here, on the stream, unless it is).
 template <int VS, bool GRID, bool INL, int SAFE = 0>
 cudaError_t batch_cells(const CellLaunch *descs, const int *start, int ndiag, const Layout &L, int only_status,
                         const int *park_counter, int park_capacity, long rows, int *work, cudaStream_t st,
-                        int sm_count, const int *left = nullptr) {
+                        int sm_count, const int *left = nullptr, int below = INT_MAX, bool zeroed = false) {
   const int wpb = warps_per_block_for(L);
   if (wpb == 0) return cudaErrorInvalidValue;
   const size_t smem = size_t(L.total) * wpb;
@@ -3364,9 +3366,9 @@ cudaError_t batch_cells(const CellLaunch *descs, const int *start, int ndiag, co
     work = nullptr;
   } else {
     blocks = resident_blocks(k, wpb * 32, smem, sm_count);
-    if (work && (e = cudaMemsetAsync(work, 0, sizeof(int), st)) != cudaSuccess) return e;
+    if (work && !zeroed && (e = cudaMemsetAsync(work, 0, sizeof(int), st)) != cudaSuccess) return e;
   }
-  k<<<blocks, wpb * 32, smem, st>>>(descs, start, ndiag, L, only_status, park_counter, park_capacity, left, work);
+  k<<<blocks, wpb * 32, smem, st>>>(descs, start, ndiag, L, only_status, park_counter, park_capacity, left, below, work);
   return cudaGetLastError();
 }
 

@@ -79,7 +79,7 @@ cudaError_t batch_clip_ahead(const CellBatch &b, const CellLaunch *descs, const 
     work = b.work;
     if ((e = cudaMemsetAsync(work, 0, sizeof(int), st)) != cudaSuccess) return e;
   }
-  k<<<blocks, threads, smem, st>>>(descs, start, b.ndiag, O, work);
+  k<<<blocks, threads, smem, st>>>(descs, start, b.ndiag, O, rows >= 0 ? 0 : kOctetMinRows, work);
   return cudaGetLastError();
 }
 
@@ -102,6 +102,29 @@ cudaError_t batch_finish(const CellBatch &b, const CellLaunch *descs, const Layo
   return cudaGetLastError();
 }
 
+// The cells of a launch: with eight lanes each (their records are left), or
+// of few rows with a warp each.  Where only the device knows the rows
+// (rows < 0) both kernels are launched and one of them does nothing.
+template <int VS, bool GRID, bool INL>
+cudaError_t batch_rows(const CellBatch &b, const CellLaunch *descs, const int *start, long rows, const Layout &L,
+                       cudaStream_t st, int sm_count, int &n) {
+  cudaError_t e;
+  const bool some = rows < 0;
+  if (some || rows >= kOctetMinRows) {
+    e = b.P <= 32 ? batch_clip<1, GRID>(b, descs, start, rows, st, sm_count)
+                  : batch_clip<2, GRID>(b, descs, start, rows, st, sm_count);
+    if (e != cudaSuccess) return e;
+    ++n;
+  }
+  if (some || rows < kOctetMinRows) {
+    if ((e = batch_cells<VS, GRID, INL>(descs, start, b.ndiag, L, -1, nullptr, 0, rows, b.work, st, sm_count, nullptr,
+                                        kOctetMinRows, some)) != cudaSuccess)
+      return e;
+    ++n;
+  }
+  return cudaSuccess;
+}
+
 // The plain diagrams' cells (no domain), then those with one; the records of
 // each are finished, and the cells left over re-run with a warp each, before
 // the next use of the counters.
@@ -113,26 +136,26 @@ cudaError_t launch_batch_octet_vs(const CellBatch &b, const Layout &Lg, const La
   int n = 0;
   if (b.start_plain) {
     if ((e = cudaMemsetAsync(b.hand.ctr, 0, ctr_bytes, st)) != cudaSuccess) return e;
-    e = b.P <= 32 ? batch_clip<1, false>(b, b.descs_inline, b.start_plain, b.rows_plain, st, sm_count)
-                  : batch_clip<2, false>(b, b.descs_inline, b.start_plain, b.rows_plain, st, sm_count);
-    if (e != cudaSuccess) return e;
+    if ((e = batch_rows<VS, false, true>(b, b.descs_inline, b.start_plain, b.rows_plain, Lp, st, sm_count, n)) !=
+        cudaSuccess)
+      return e;
     if (b.HC && (e = batch_finish<VS, false, true>(b, b.descs_inline, Lp, st, sm_count)) != cudaSuccess) return e;
     if ((e = batch_cells<VS, false, true>(b.descs_inline, b.start_plain, b.ndiag, Lp, kParkOverflow, nullptr, 0, -1,
                                           b.work, st, sm_count, b.hand.ctr + 2)) != cudaSuccess)
       return e;
-    n += 2 + (b.HC ? 1 : 0);
+    n += 1 + (b.HC ? 1 : 0);
   }
   if (b.start_grid) {
     const bool park = b.defer.slots != nullptr;
     const CellLaunch *descs = park ? b.descs : b.descs_inline;
     if ((e = cudaMemsetAsync(b.hand.ctr, 0, ctr_bytes, st)) != cudaSuccess) return e;
-    e = b.P <= 32 ? batch_clip<1, true>(b, descs, b.start_grid, b.rows_grid, st, sm_count)
-                  : batch_clip<2, true>(b, descs, b.start_grid, b.rows_grid, st, sm_count);
+    e = park ? batch_rows<VS, true, false>(b, descs, b.start_grid, b.rows_grid, Lg, st, sm_count, n)
+             : batch_rows<VS, true, true>(b, descs, b.start_grid, b.rows_grid, Lg, st, sm_count, n);
     if (e != cudaSuccess) return e;
     e = park ? batch_finish<VS, true, false>(b, descs, Lg, st, sm_count)
              : batch_finish<VS, true, true>(b, descs, Lg, st, sm_count);
     if (e != cudaSuccess) return e;
-    n += 2;
+    ++n;
     if ((e = record_after_cell(b, st)) != cudaSuccess) return e;
     if (park) {
       if ((e = launch_cones_batch<VS>(b, Lg, st, sm_count)) != cudaSuccess) return e;

@@ -892,15 +892,17 @@ __global__ void __launch_bounds__(128, MW == 1 && !AHEAD ? 6 : 5)
 
 // The rows of many diagrams (k_cell_batch's scheme): diagram d owns rows
 // start[d] .. start[d+1].  work (optional, zeroed before the launch): warps
-// take four rows at a time from it; null: one octet per row.
+// take four rows at a time from it; null: one octet per row.  from: launches
+// of fewer rows are another kernel's.
 template <int MW, bool GRID, bool AHEAD>
 __global__ void __launch_bounds__(128, 5)
     k_clip_batch(const CellLaunch *__restrict__ descs, const int *__restrict__ start, int ndiag,
-                 const __grid_constant__ OctLayout L, int *__restrict__ work) {
+                 const __grid_constant__ OctLayout L, int from, int *__restrict__ work) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int lane = threadIdx.x & 31;
   unsigned char *osm = smem + size_t(threadIdx.x / kOct) * L.total;
   const int total = start[ndiag];
+  if (total < from) return;
   int r0 = (blockIdx.x * blockDim.x + threadIdx.x) / 32 * 4;
   for (;;) {
     if (work) {

@@ -664,13 +664,6 @@ int knn_variant_for(rpd_solver *s, const int *ids, int num, int K, unsigned *out
   return ctx->knn_last[K] = choice;
 }
 
-// Launches of fewer rows clip with a warp per cell: an octet's cell takes
-// longer than a warp's, which only more cells at a time repay (uniform seeds,
-// K 50, octet / warp: 2,000 rows 0.102 / 0.076 ms in the box and 0.145 /
-// 0.122 in a cube domain, 4,000 rows 0.109 / 0.127 and 0.156 / 0.189, 16,000
-// rows 0.205 / 0.377 and 0.295 / 0.547).
-constexpr int kOctetMinRows = 4096;
-
 // One pass (VoroAlgoComputeData::launch, voronoi.cpp:861-1036): the K
 // nearest of the listed seeds, then their cells with this pass's caps.
 static_assert(int(RPD_CTR_NUM) == int(kCtrNum), "counter enums out of sync");
