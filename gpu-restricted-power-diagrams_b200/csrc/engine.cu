@@ -681,8 +681,11 @@ int run_pass(rpd_solver *s, const int *ids, int num, int K, int P, int V, int T,
   const bool all_cells = ids == nullptr && num == s->n;
   rpd::DevBuf &kb = all_cells ? s->knn : s->knn_part;
   const bool ahead_first = s->ahead_on && pi == 0;
-  const int Kx = ahead_first ? ahead_columns(K) : retry_K > 0 ? retry_K : K;
-  const bool reuse = all_cells && s->knn_full_K == K && s->knn_full_Kx == Kx && !counters && !s->fresh_knn;
+  int Kx = ahead_first ? ahead_columns(K) : retry_K > 0 ? retry_K : K;
+  // longer rows than a launch needs hold its lists too (Newton steps with
+  // Hessian rows and the solves between them alternate at K <= 24)
+  const bool reuse = all_cells && s->knn_full_K == K && s->knn_full_Kx >= Kx && !counters && !s->fresh_knn;
+  if (reuse) Kx = s->knn_full_Kx;
   if ((e = kb.ensure(sizeof(unsigned) * size_t(num) * Kx)) != cudaSuccess) return map_cuda(ctx, e, "alloc knn");
   Events<4> ev;
   unsigned long long *ctr = counters ? s->counter64.as<unsigned long long>() : nullptr;
