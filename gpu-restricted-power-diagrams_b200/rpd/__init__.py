@@ -245,7 +245,20 @@ class Context:
         self.h = lib().rpd_context_create(device, C.byref(err))
         if not self.h:
             raise RpdError(err.value, f"no usable sm_100 device {device}")
+        # handles of solvers and batches on this context and what destroys
+        # them: the collector may close a context before them (a cycle, such
+        # as a traceback's, that holds them all), and they need it to go
+        self._owned = {}
         _track("context", self)
+
+    def _own(self, handle, destroy: str):
+        self._owned[handle] = destroy
+
+    def _destroy(self, handle):
+        """Destroys a handle of this context, once."""
+        destroy = self._owned.pop(handle, None)
+        if destroy:
+            getattr(lib(), destroy)(handle)
 
     def error(self) -> str:
         return lib().rpd_context_error(self.h).decode()
@@ -264,6 +277,8 @@ class Context:
 
     def close(self):
         if self.h:
+            for handle in reversed(list(self._owned)):
+                self._destroy(handle)
             lib().rpd_context_destroy(self.h)
             self.h = None
 
@@ -328,6 +343,7 @@ class Solver:
         self.h = lib().rpd_solver_create(self.ctx.h, C.byref(err))
         if not self.h:
             raise RpdError(err.value, self.ctx.error())
+        self.ctx._own(self.h, "rpd_solver_destroy")
         _track("solver", self)
 
     def set_points(self, xyzw):
@@ -504,7 +520,7 @@ class Solver:
 
     def close(self):
         if self.h:
-            lib().rpd_solver_destroy(self.h)
+            self.ctx._destroy(self.h)
             self.h = None
 
     def __del__(self):
@@ -580,6 +596,7 @@ class Batch:
         if not self.h:
             raise RpdError(err.value, self.ctx.error())
         self._keep = (hs, pa)
+        self.ctx._own(self.h, "rpd_batch_destroy")
         _track("batch", self)
 
     def launch(self):
@@ -593,7 +610,7 @@ class Batch:
 
     def close(self):
         if self.h:
-            lib().rpd_batch_destroy(self.h)
+            self.ctx._destroy(self.h)
             self.h = None
 
     def __del__(self):
