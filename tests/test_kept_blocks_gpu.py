@@ -1,51 +1,50 @@
 """Freed device blocks kept for reuse, beside a server's memory budget: when a
-request is admitted, those that do not fit beside it are given back."""
-import gc
+request is admitted, those that do not fit beside it are given back.  In a
+process of its own, whose device memory is what it allocated."""
+import os
+import subprocess
+import sys
 
-import numpy as np
 import pytest
 
 pytestmark = pytest.mark.gpu
 
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 MB = 1 << 20
 
+PROGRAM = """
+import numpy as np, rpd, sys
+from cuda.bindings import runtime as rt
+from rpd import synth
 
-@pytest.fixture(scope="module")
-def rpd():
-    torch = pytest.importorskip("torch")
-    if not torch.cuda.is_available():
-        pytest.skip("no GPU")
-    import rpd as m
-
-    return m
-
-
-def pool_used():
-    """Bytes that allocations hold of the device's memory pool, the kept
-    blocks among them."""
-    from cuda.bindings import runtime as rt
-
+def pool_used():  # bytes that allocations hold of the device's memory pool, the kept blocks among them
     err, pool = rt.cudaDeviceGetDefaultMemPool(0)
     err, used = rt.cudaMemPoolGetAttribute(pool, rt.cudaMemPoolAttr.cudaMemPoolAttrUsedMemCurrent)
     return int(used)
 
+ctx = rpd.Context(0)
+s = rpd.Solver(ctx).set_points(synth.uniform(2_000_000, seed=1))
+s.launch(K=70, P=30, V=40)
+s.close()
+print(pool_used())  # kept: the context is alive
+x = synth.uniform(20_000, seed=2)
+with rpd.Server(slots=2, mem_budget=int(sys.argv[1])) as sv:
+    for _ in range(3):
+        t, session = sv.solve(x, K=50, P=30, V=40)
+        assert np.isfinite(sv.wait(t)[0]).all()
+        print(pool_used())
+    print(sv.bytes_in_use())
+"""
 
-@pytest.mark.parametrize("budget", [128, 512])
-def test_kept_blocks_within_the_budget(rpd, budget):
-    from rpd import synth
 
-    gc.collect()
-    ctx = rpd.Context(0)
-    before = pool_used()
-    s = rpd.Solver(ctx).set_points(synth.uniform(2_000_000, seed=1))
-    s.launch(K=70, P=30, V=40)
-    s.close()
-    assert pool_used() - before > 700 * MB  # kept: the context is alive
-    x = synth.uniform(20_000, seed=2)
-    with rpd.Server(slots=2, mem_budget=budget * MB) as sv:
-        for _ in range(3):
-            t, session = sv.solve(x, K=50, P=30, V=40)
-            assert np.isfinite(sv.wait(t)[0]).all()
-            assert pool_used() - before <= budget * MB
-        assert sv.bytes_in_use() <= budget * MB
-    ctx.close()
+@pytest.mark.parametrize("budget", [128 * MB, 512 * MB])
+def test_kept_blocks_within_the_budget(budget):
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("no GPU")
+    env = dict(os.environ, PYTHONPATH=os.path.join(ROOT, "gpu-restricted-power-diagrams_b200"))
+    out = subprocess.run([sys.executable, "-c", PROGRAM, str(budget)], env=env, capture_output=True, text=True, timeout=300)
+    assert out.returncode == 0, out.stderr
+    kept, *held = [int(v) for v in out.stdout.split()]
+    assert kept > 700 * MB
+    assert max(held) <= budget
