@@ -19,7 +19,8 @@ constexpr int kMaxDev = 64;
 std::mutex g_alloc_mu;
 cudaStream_t g_alloc_stream[kMaxDev] = {};
 
-// Freed blocks by size class (never destroyed: buffers may outlive statics).
+// Freed blocks by size, no list empty (never destroyed: buffers may outlive
+// statics).
 struct Kept {
   std::mutex mu;
   std::map<size_t, std::vector<void *>> blocks;
@@ -27,7 +28,9 @@ struct Kept {
   int contexts = 0;
 };
 Kept *const g_kept = new Kept[kMaxDev];
-constexpr size_t kKeepBlock = size_t(1) << 30;
+constexpr size_t kKeepBlock = size_t(4) << 30;
+
+constexpr size_t kMostSlack = 2;  // a kept block of up to so many times the size asked for serves
 
 size_t size_class(size_t bytes) {
   size_t step = 512;
@@ -60,22 +63,16 @@ void pool_trim(int dev, size_t most) {
   std::lock_guard<std::mutex> lock(k.mu);
   cudaStream_t st;
   if (k.bytes <= most || alloc_stream(dev, &st) != cudaSuccess) return;
-  while (k.bytes > most && !k.blocks.empty()) {
+  while (k.bytes > most) {
     const auto c = std::prev(k.blocks.end());  // the largest first
-    if (!c->second.empty()) {
-      cudaFreeAsync(c->second.back(), st);
-      c->second.pop_back();
-      k.bytes -= c->first;
-    }
+    cudaFreeAsync(c->second.back(), st);
+    c->second.pop_back();
+    k.bytes -= c->first;
     if (c->second.empty()) k.blocks.erase(c);
   }
 }
 
-size_t pool_block(size_t bytes) {
-  return bytes > 0 && bytes <= pool_detail::kKeepBlock ? pool_detail::size_class(bytes) : bytes;
-}
-
-cudaError_t pool_alloc(void **p, size_t bytes, int *device) {
+cudaError_t pool_alloc(void **p, size_t bytes, size_t *block, int *device) {
   using namespace pool_detail;
   int dev = 0;
   cudaStream_t st;
@@ -83,16 +80,20 @@ cudaError_t pool_alloc(void **p, size_t bytes, int *device) {
   if (e != cudaSuccess || (e = alloc_stream(dev, &st)) != cudaSuccess) return e;
   *device = dev;
   if (bytes <= kKeepBlock) {
-    bytes = pool_block(bytes);
-    std::lock_guard<std::mutex> lock(g_kept[dev].mu);
-    auto c = g_kept[dev].blocks.find(bytes);
-    if (c != g_kept[dev].blocks.end() && !c->second.empty()) {
+    bytes = size_class(bytes);
+    Kept &k = g_kept[dev];
+    std::lock_guard<std::mutex> lock(k.mu);
+    const auto c = k.blocks.lower_bound(bytes);
+    if (c != k.blocks.end() && c->first <= bytes * kMostSlack) {
       *p = c->second.back();
+      *block = c->first;
       c->second.pop_back();
-      g_kept[dev].bytes -= bytes;
+      k.bytes -= c->first;
+      if (c->second.empty()) k.blocks.erase(c);
       return cudaSuccess;
     }
   }
+  *block = bytes;
   if ((e = cudaMallocAsync(p, bytes, st)) == cudaErrorMemoryAllocation) {
     cudaGetLastError();
     pool_trim(dev, 0);
@@ -103,17 +104,20 @@ cudaError_t pool_alloc(void **p, size_t bytes, int *device) {
   return cudaStreamSynchronize(st);
 }
 
-void pool_free(void *p, size_t bytes, int dev) {
+void pool_free(void *p, size_t block, int dev) {
   using namespace pool_detail;
-  if (bytes <= kKeepBlock) {
-    bytes = pool_block(bytes);
-    std::lock_guard<std::mutex> lock(g_kept[dev].mu);
-    if (g_kept[dev].contexts > 0 && g_kept[dev].bytes + bytes <= g_kept[dev].most) {
+  if (block <= kKeepBlock) {
+    Kept &k = g_kept[dev];
+    std::lock_guard<std::mutex> lock(k.mu);
+    if (k.contexts > 0 && k.bytes + block <= k.most) {
+      auto c = k.blocks.end();
       try {
-        g_kept[dev].blocks[bytes].push_back(p);
-        g_kept[dev].bytes += bytes;
+        c = k.blocks.try_emplace(block).first;
+        c->second.push_back(p);
+        k.bytes += block;
         return;
       } catch (const std::bad_alloc &) {  // then to the driver's pool
+        if (c != k.blocks.end() && c->second.empty()) k.blocks.erase(c);
       }
     }
   }
@@ -128,7 +132,7 @@ void pool_context(int dev, int change, size_t device_bytes) {
   {
     std::lock_guard<std::mutex> lock(g_kept[dev].mu);
     g_kept[dev].contexts += change;
-    if (device_bytes) g_kept[dev].most = device_bytes / 32;
+    if (device_bytes) g_kept[dev].most = device_bytes / 16;
     last = g_kept[dev].contexts <= 0;
   }
   if (last) pool_trim(dev, 0);
@@ -1820,7 +1824,7 @@ size_t solver_device_bytes(const rpd_solver *s) {
                        &s->ids_c, &s->fail_ws, &s->hist, &s->gather, &s->defer_slots, &s->defer_part, &s->defer_fail,
                        &s->defer_ctr, &s->defer_chunk_slot, &s->hand_recs, &s->hand_ctr, &s->ahead, &s->wmin, &s->used, &s->hess, &s->hessid};
   size_t t = 0;
-  for (const DevBuf *x : b) t += pool_block(x->bytes);
+  for (const DevBuf *x : b) t += x->block;
   return t;
 }
 

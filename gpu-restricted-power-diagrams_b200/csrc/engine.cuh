@@ -20,39 +20,43 @@ namespace rpd {
 // work that uses it is pending: every entry point of the engine ends with a
 // synchronization of its stream.
 //
-// Freed blocks of up to 1 GB are kept by size class (eight steps per power of
-// two, so up to 1/8 of a block is unused) and handed out again without a call
-// into the driver, up to 1/32 of the device's memory while a context of the
-// device exists; the serving loop gives back what its budget does not hold
-// (pool_trim).  The driver's pool alone puts a large block together from
-// fragments where freed blocks of other sizes lie in between; that took 10 to
-// 160 ms each (192 MB of parked cells' slots) and stopped all streams: twelve
-// requests on four streams took 0.1 to 1.5 s instead of 50 ms in one burst of
-// eight.
-cudaError_t pool_alloc(void **p, size_t bytes, int *device);
-void pool_free(void *p, size_t bytes, int device);
+// Freed blocks of up to 4 GB are kept and handed out again without a call
+// into the driver: the smallest one that holds the bytes, if it is at most
+// twice as large; up to 1/16 of the device's memory while a context of the
+// device exists.  The serving loop gives back what its budget does not hold
+// (pool_trim).  The driver's pool puts a large block together from fragments
+// where freed blocks of other sizes lie in between, or maps new memory; that
+// takes 10 ms to a second and stops all streams.  600 served requests of 10K
+// to 2M seeds on four streams, four runs each: with blocks kept by exact size
+// class 1,900 calls into the driver, 6 to 14 s in the slow ones, 27 to 28M
+// cells/s; now 900, 0.2 to 0.4 s, 33.5M; with blocks of up to 1.5 times 680
+// (1/8 of the memory), 2 s.  Half that load, p50 / p99: 13 / 110 to 570 ms ->
+// 13 / 55.  Everything to the driver's pool, the kernels before: 19M cells/s,
+// 24 / 114 ms.
+cudaError_t pool_alloc(void **p, size_t bytes, size_t *block, int *device);
+void pool_free(void *p, size_t block, int device);
 void pool_context(int device, int change, size_t device_bytes = 0);  // a context made (1) or destroyed (-1)
 // Gives kept blocks back to the driver's pool until at most `most` bytes are kept.
 void pool_trim(int device, size_t most);
-size_t pool_block(size_t bytes);  // the block's size for an allocation of `bytes`
 
 struct DevBuf {
   void *ptr = nullptr;
   size_t bytes = 0;
-  int device = 0;  // the block's
+  size_t block = 0;  // the size of the block that holds them
+  int device = 0;    // the block's
   DevBuf() = default;
   DevBuf(const DevBuf &) = delete;
   DevBuf &operator=(const DevBuf &) = delete;
   ~DevBuf() { release(); }
   void release() {
-    if (ptr) pool_free(ptr, bytes, device);
+    if (ptr) pool_free(ptr, block, device);
     ptr = nullptr;
-    bytes = 0;
+    bytes = block = 0;
   }
   cudaError_t ensure(size_t want) {
     if (want <= bytes && ptr) return cudaSuccess;
     release();
-    cudaError_t e = pool_alloc(&ptr, want ? want : 16, &device);
+    cudaError_t e = pool_alloc(&ptr, want ? want : 16, &block, &device);
     if (e == cudaSuccess) bytes = want ? want : 16;
     else ptr = nullptr;
     return e;
