@@ -503,6 +503,7 @@ __device__ __forceinline__ void clip_octet(const CellLaunch &a, const OctLayout 
     }
   }
   const bool work = run;  // the octet has a cell to clip
+  bool reclip = false;    // left to the warp kernel: the caps here do not hold the cell, or its seed
   // the neighbours' ids, a chunk ahead of their use
   unsigned zn = kNone;
   const bool ahead = AHEAD && work && a.ahead && a.ahead_first;
@@ -519,7 +520,20 @@ __device__ __forceinline__ void clip_octet(const CellLaunch &a, const OctLayout 
   }
   int vst = -1;  // the status under the caps, once one of them is passed
   // the domain box
-  if (l8 < 6) plane[l8] = box_plane(s, work ? a.cube_eps : 0.f, l8);
+  {
+    bool out = false;
+    if (l8 < 6) {
+      const Plane p = box_plane(s, work ? a.cube_eps : 0.f, l8);
+      plane[l8] = p;
+      out = p.w < 0.0;
+    }
+    // a seed outside the box: clipped to its end its cell may be empty, where
+    // the warp kernel has proven it outside the domain before (a success)
+    if (GRID && oct_bits(out) && run) {
+      reclip = true;
+      run = false;
+    }
+  }
   __syncwarp();
   {
     // its corners: exact, the planes being axis-parallel
@@ -533,7 +547,6 @@ __device__ __forceinline__ void clip_octet(const CellLaunch &a, const OctLayout 
   int np = 6, nv = 8;
   const int Pm = !work ? 0 : (ahead ? L.Pc : min(a.P, kOctP));
   const int Vm = ahead ? L.Vc : min(a.V, kOctV);
-  bool reclip = false;    // the caps here do not hold the cell: the warp kernel clips it
   bool inside = false;    // the seed surely lies in its own cell (nonempty_cell)
   bool cut = false;
   int i0 = -kOct, jj = kOct;  // neighbour i0 + jj comes next (jj == kOct: the next chunk's first)
