@@ -259,11 +259,12 @@ size_t defer_slot_bytes(int P, int V, int T);
 // k_cell over the rows; with a domain and a defer queue, also the chunked
 // boundary-triangle kernel and the per-cell reduction (3 launches).
 cudaError_t cell_launch(const CellLaunch &a, cudaStream_t st, int sm_count = 148, int *launches = nullptr);
+// The same with eight lanes per cell (a.hand.recs; cell_octet.cu), and whether
+// a launch's cells can be clipped so.
+cudaError_t cell_launch_octet(const CellLaunch &a, cudaStream_t st, int sm_count, int *launches);
+bool octet_applies(const CellLaunch &a);
 // The same for a.precision > 0 (cell_prec.cu), and for FP64 clipping with
 // the weighted security-radius guard (a.safe_radius; cell_safe.cu).
-cudaError_t cell_launch_octet(const CellLaunch &a, cudaStream_t st, int sm_count, int *launches);
-// Whether a launch's cells can be clipped with eight lanes each.
-bool octet_applies(const CellLaunch &a);
 cudaError_t cell_launch_prec(const CellLaunch &a, cudaStream_t st, int sm_count, int *launches);
 cudaError_t cell_launch_safe(const CellLaunch &a, cudaStream_t st, int sm_count, int *launches);
 
@@ -327,7 +328,8 @@ struct CellBatch {
   bool ahead = false;     // a first pass with diagrams that clip past their caps (CellLaunch::ahead)
 };
 cudaError_t cell_batch_launch(const CellBatch &b, cudaStream_t st, int sm_count, int *launches = nullptr);
-// The same with the guard compiled in (cell_safe.cu).
+// The same with eight lanes per cell where the rows are many (b.hand.recs;
+// cell_octet.cu), and with the guard compiled in (cell_safe.cu).
 cudaError_t cell_batch_launch_octet(const CellBatch &b, cudaStream_t st, int sm_count, int *launches);
 cudaError_t cell_batch_launch_safe(const CellBatch &b, cudaStream_t st, int sm_count, int *launches);
 

@@ -1,7 +1,8 @@
 // Device code of the restricted cell kernels, included by the translation
-// units that instantiate them: cell.cu (FP64 clipping, batched solves, the
-// outside probe, the cone kernels) and cell_prec.cu (the FP32 clipping
-// variants), so the two compile in parallel.
+// units that instantiate them, which compile in parallel: cell.cu (FP64
+// clipping with a warp per cell, batches of few rows, the outside probe),
+// cell_octet.cu (through clip_octet.cuh: eight lanes per cell), cell_prec.cu
+// (the FP32 clipping variants) and cell_safe.cu (the radius guard).
 #pragma once
 // Restricted power cell of every seed, one warp per cell.  Replaces the
 // reference's one-work-item compute_voro_cell (ConvexCell.cl:812-1116).

@@ -9,9 +9,9 @@
 // made, the cavity has 3 to 10 triangles).  With eight lanes per cell the
 // same instructions serve four cells: 4.6K warp instructions per cell instead
 // of 8.8K on 1M weighted lattice seeds in a blob (K 50), first pass 15.8 ->
-// 6.5 ms with the finish kernel; 2M blue-noise seeds (K 20, P 25, V 30) 32.5
-// -> 10.0 ms.  What bounds it: instruction issue (2.5 of 4 per cycle) and
-// instruction fetch -- the loop's code is kept small (seldom taken loops
+// 7.1 ms with the finish kernel (6.1 + 1.0); 2M blue-noise seeds (K 20, P 25,
+// V 30) 32.5 -> 10.0 ms.  What bounds it: instruction issue (2.67 of 4 per
+// cycle) and instruction fetch -- the loop's code is kept small (seldom taken loops
 // rolled, the end of a cell out of line): 8.4 -> 6.8 ms by that alone.
 // Five or six blocks per SM, by registers (96 / 80) and shared memory (2.2 KB
 // per cell at P 30, V 40); sixteen lanes would serve two cells only, four
