@@ -211,12 +211,12 @@ __device__ __forceinline__ void merge_row(const float4 *__restrict__ stored, con
 // up to T are sorted.  The list is merge_row's bit for bit: T lies where no
 // seed outside the shells that merge_row scans, or outside the block, can be,
 // so the K least keys are the same keys.  Measured against merge_row alone,
-// 300K uniform seeds: 1.01 -> 0.61 ms at K 50, 0.74 -> 0.48 at K 20, 2.07 ->
-// 1.39 at K 96; 1M lattice seeds at K 50 3.26 -> 1.90.  A row that is not
+// 300K uniform seeds: 1.00 -> 0.60 ms at K 50, 0.73 -> 0.46 at K 20, 2.05 ->
+// 1.38 at K 96; 1M lattice seeds at K 50 3.26 -> 1.90.  A row that is not
 // decided costs both: with the third shell's bound in place of the block's
 // face most rows of K 96 and those near the box's faces did (1.87 ms), and
 // with a fall-through where K lie below the second shell's bound those of K
-// <= 13 (K 8: 0.49 -> 0.69, now 0.44).  Up to K 6 the scan of 84 candidates
+// <= 13 (K 8: 0.48 -> 0.67, now 0.43).  Up to K 6 the scan of 84 candidates
 // is the faster (K 1: 0.40 against 0.43 ms).  Seeds in dense clusters, whose
 // blocks hold more candidates than registers, pay 3 to 4%.
 constexpr int kSelectSlots = 3;    // K <= 96
@@ -323,19 +323,24 @@ __device__ __forceinline__ bool select_row(const float4 *__restrict__ stored, co
     if (below(__float_as_uint(b * b)) != ch) return false;
   } else {
     // merge_row scans shell 2, and further ones as long as fewer than K lie
-    // below their bounds; none of those holds a nearer candidate than the
-    // nearest face of the block with bins beyond
-    float face = 5.f * w;
-    if (cx > 2) face = fminf(face, p.x - float(cx - 2) * w);
-    if (cy > 2) face = fminf(face, p.y - float(cy - 2) * w);
-    if (cz > 2) face = fminf(face, p.z - float(cz - 2) * w);
-    if (cx + 3 < dim) face = fminf(face, float(cx + 3) * w - p.x);
-    if (cy + 3 < dim) face = fminf(face, float(cy + 3) * w - p.y);
-    if (cz + 3 < dim) face = fminf(face, float(cz + 3) * w - p.z);
-    face = fmaxf(face - kFaceErr, 0.f);
-    t = __float_as_uint(fmaxf(face * face, __ldg(&ring_bound[3])));
+    // below their bounds
+    t = __float_as_uint(__ldg(&ring_bound[3]));
     ch = below(t);
-    if (ch < K) return false;
+    if (ch < K) {
+      // none of those holds a nearer candidate than the nearest face of the
+      // block with bins beyond
+      float face = 5.f * w;
+      if (cx > 2) face = fminf(face, p.x - float(cx - 2) * w);
+      if (cy > 2) face = fminf(face, p.y - float(cy - 2) * w);
+      if (cz > 2) face = fminf(face, p.z - float(cz - 2) * w);
+      if (cx + 3 < dim) face = fminf(face, float(cx + 3) * w - p.x);
+      if (cy + 3 < dim) face = fminf(face, float(cy + 3) * w - p.y);
+      if (cz + 3 < dim) face = fminf(face, float(cz + 3) * w - p.z);
+      face = fmaxf(face - kFaceErr, 0.f);
+      t = __float_as_uint(face * face);
+      ch = below(t);
+      if (ch < K) return false;
+    }
   }
   if (ch > kMost) {
     unsigned lo = 0, hi = t;
