@@ -770,6 +770,10 @@ int capture(rpd_batch *b) {
     long long all = 0;
     for (int d = 0; d < nd; ++d) all += G[d].H > 0 ? G[d].n : 0;
     hand.capacity = int(std::min(cells, clip_hand_capacity(int(cells)) + all));
+    if (all > 0 && b->hand_recs.ensure(size_t(kClipRecordBytes) * hand.capacity) != cudaSuccess) {
+      cudaGetLastError();  // the smaller array will do
+      hand.capacity = clip_hand_capacity(int(cells));
+    }
     if ((e = b->hand_recs.ensure(size_t(kClipRecordBytes) * hand.capacity)) != cudaSuccess ||
         (e = b->hand_ctr.ensure(sizeof(int) * kClipCounters)) != cudaSuccess)
       return map_cuda(ctx, e, "alloc batch clip records");
